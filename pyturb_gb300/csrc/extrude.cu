@@ -17,6 +17,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <map>
 #include <vector>
@@ -603,6 +604,295 @@ __global__ void k_extrude_reduce(int W, int J, int cap, int nsplit, const float*
   slab[(size_t)dst.d[j].y * W + r] = s;
 }
 
+// ---------------------------------------------------------------- few screens
+// A row step of a handful of screens (one atmosphere's layers, or one infinite
+// screen) is a matrix-vector sized product: its cost as gather, split-K GEMM,
+// reduce, anchor GEMM and anchor apply was five launches' latency, 27 us of
+// device time for 9 layers at W = 728 and as much again on the host. Two
+// launches do it here. k_row_step: a CTA owns RT consecutive new pixels (or a
+// few such groups), stages every job's operand in shared memory straight from
+// the rings, its warps split K, and the sums end in the ring without slices in
+// memory; the CTA also adds its share of the anchor's projections (a slice of
+// the operand columns, and its own new pixels) and makes its share of the next
+// launch's noise. k_step_anchor sums the shares and corrects the rows. So the
+// same step takes 11 us + 5 us (both latency: the operand's way through L2, the
+// reduction, the anchor's double-float chains). More than kStepJobs screens, or
+// an operand beyond shared memory, leave the product to the tiled GEMM, which
+// reuses each operator value for 32 jobs and more.
+constexpr int kStepJobs = 16;
+constexpr int kStepThreads = 512;
+constexpr int kStepWarps = kStepThreads / 32;
+constexpr int kStepUnroll = 4;  // operand columns of a lane in flight
+
+struct StepJobs {
+  int n;
+  int screen[kStepJobs], head[kStepJobs];
+  float bscale[kStepJobs];
+  uint64_t key[kStepJobs], row[kStepJobs];
+  long long noise_off[kStepJobs];
+};
+
+// scaled noise of the jobs, out[j][c]: thread `t` of `total` makes its share of
+// column pairs (the values of k_extrude_gather)
+__device__ __forceinline__ void step_noise(const StepJobs& jobs, int W, const float* __restrict__ inject,
+                                           float* __restrict__ out, int t, int total) {
+  const int half = (W + 1) / 2;
+  for (int e = t; e < jobs.n * half; e += total) {
+    const int j = e / half, c = 2 * (e - j * half);
+    float2 z;
+    if (inject) {
+      const float* src = inject + jobs.noise_off[j] + c;
+      z = make_float2(src[0], c + 1 < W ? src[1] : 0.f);
+    } else {
+      z = philox_cnormal(jobs.key[j], (uint64_t)(c >> 1), jobs.row[j], kDomainExtrude);
+    }
+    out[(size_t)j * W + c] = jobs.bscale[j] * z.x;
+    if (c + 1 < W) out[(size_t)j * W + c + 1] = jobs.bscale[j] * z.y;
+  }
+}
+
+__global__ void __launch_bounds__(256)
+k_step_noise(const StepJobs jobs, int W, const float* __restrict__ inject, float* __restrict__ out) {
+  step_noise(jobs, W, inject, out, blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x);
+}
+
+// One halving of the warp sum of N values a lane: lanes with bit O of the lane
+// index take the upper half of the values, the others the lower.
+template <int N, int O>
+__device__ __forceinline__ void warp_halve(float* v, int lane) {
+  const bool up = lane & O;
+#pragma unroll
+  for (int i = 0; i < N / 2; ++i) {
+    const float keep = up ? v[i + N / 2] : v[i], give = up ? v[i] : v[i + N / 2];
+    v[i] = keep + __shfl_xor_sync(0xffffffffu, give, O);
+  }
+}
+
+struct StepArgs {
+  int W, m, cap, K, Kz, rows;  // rows of the new row a CTA makes
+  const float* M;              // (W, K) of the jobs' group
+  float* buf;
+  const float* noise;          // (J, W) scaled noise of this launch
+  const float* inject;         // the caller's noise, or NULL (Philox)
+  float* noise_next;           // the next launch's
+  const f2p* th;               // anchor tables of the group, or NULL
+  const f2p* tl;
+  int np2;                     // mode pairs
+  int kslice;                  // operand columns of a CTA's anchor share
+  float2* part;                // (J, 2 CTAs, 2 np2) shares
+};
+
+template <int RT, int JT>
+__global__ void __launch_bounds__(kStepThreads, 1)
+k_row_step(const StepArgs a, const StepJobs jobs, const StepJobs next) {
+  extern __shared__ float xs[];  // (J, K) operand
+  constexpr int NV = RT * JT, NP = (NV + 31) / 32 * 32;
+  __shared__ float red[kStepWarps][NP + 1];
+  float* newrow = xs + (size_t)jobs.n * a.K;  // (J, rows)
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int W = a.W, K = a.K, J = jobs.n;
+  const int rbeg = blockIdx.x * a.rows, rend = min(W, rbeg + a.rows);
+  // operand: m ring rows and the noise row of every job
+  for (int j = 0; j < J; ++j) {
+    const float* slab = a.buf + (size_t)jobs.screen[j] * a.cap * W;
+    for (int r = 0; r <= a.m; ++r) {
+      const float* src = r < a.m ? slab + (size_t)ring_back(jobs.head[j], a.m - r, a.cap) * W
+                                 : a.noise + (size_t)j * W;
+      float* dst = xs + (size_t)j * K + (size_t)r * W;
+      for (int c = tid; c < W; c += kStepThreads)
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(
+                         (uint32_t)__cvta_generic_to_shared(dst + c)),
+                     "l"(src + c)
+                     : "memory");
+    }
+  }
+  asm volatile("cp.async.commit_group;" ::: "memory");
+  const uint64_t pol = l2_evict_last();  // the operator is re-read every row step
+  constexpr int step = kStepWarps * 32;
+  float mv[kStepUnroll][RT];
+  auto load = [&](int r0, int kw) {  // operator columns kw + lane, + step, ...
+#pragma unroll
+    for (int q = 0; q < RT; ++q) {
+      const float* row = a.M + (size_t)min(r0 + q, W - 1) * K + kw + lane;
+#pragma unroll
+      for (int u = 0; u < kStepUnroll; ++u)
+        mv[u][q] = kw + lane + u * step < K ? ld_keep(row + u * step, pol) : 0.f;
+    }
+  };
+  load(rbeg, warp * 32);  // travels while the operand lands
+  step_noise(next, W, a.inject, a.noise_next, blockIdx.x * kStepThreads + tid,
+             gridDim.x * kStepThreads);
+  asm volatile("cp.async.wait_group 0;" ::: "memory");
+  __syncthreads();
+  for (int r0 = rbeg; r0 < rend; r0 += RT) {
+    float acc[NP];
+#pragma unroll
+    for (int i = 0; i < NP; ++i) acc[i] = 0.f;
+    for (int kw = warp * 32; kw < K; kw += kStepUnroll * step) {
+      if (kw != warp * 32 || r0 != rbeg) load(r0, kw);
+#pragma unroll
+      for (int u = 0; u < kStepUnroll; ++u) {
+        if (kw + u * step >= K) break;  // the whole warp
+        const int k = min(kw + lane + u * step, K - 1);
+        float x[JT];
+#pragma unroll
+        for (int j = 0; j < JT; ++j) x[j] = xs[min(j, J - 1) * K + k];
+#pragma unroll
+        for (int q = 0; q < RT; ++q)
+#pragma unroll
+          for (int j = 0; j < JT; ++j) acc[q * JT + j] = fmaf(mv[u][q], x[j], acc[q * JT + j]);
+      }
+    }
+    warp_halve<NP, 16>(acc, lane);
+    warp_halve<NP / 2, 8>(acc, lane);
+    warp_halve<NP / 4, 4>(acc, lane);
+    warp_halve<NP / 8, 2>(acc, lane);
+    warp_halve<NP / 16, 1>(acc, lane);
+    // this lane's values: index i + (NP / 32) * (bits of the lane, 16 first)
+#pragma unroll
+    for (int i = 0; i < NP / 32; ++i) red[warp][lane * (NP / 32) + i] = acc[i];
+    __syncthreads();
+    if (tid < NV) {
+      const int q = tid / JT, j = tid - q * JT, r = r0 + q;
+      if (j < J && r < rend) {
+        float v = 0.f;
+#pragma unroll
+        for (int w = 0; w < kStepWarps; ++w) v += red[w][tid];
+        a.buf[((size_t)jobs.screen[j] * a.cap + jobs.head[j]) * W + r] = v;
+        newrow[j * a.rows + (r - rbeg)] = v;
+      }
+    }
+    __syncthreads();
+  }
+  if (!a.th) return;
+  // anchor shares: the table rows of operand columns [kb, ke) and of this CTA's
+  // new pixels, 2 np2 modes of every job in double-float (see k_anchor_gemm)
+  const int p = tid % a.np2, slot = tid / a.np2, slots = kStepThreads / a.np2;
+  const int j = slot % kStepJobs;
+  if (j >= J) return;
+  const int kb = blockIdx.x * a.kslice, ke = min(K, kb + a.kslice);
+  for (int h = slot / kStepJobs; h < 2; h += slots / kStepJobs) {
+    const int c0 = h == 0 ? kb : K + rbeg, c1 = h == 0 ? ke : K + rend;
+    f2p s = 0ull, c = 0ull;
+    for (int kc = c0; kc < c1; kc += 8) {  // table entries in flight, 8 columns at a time
+      f2p ah[8], al[8];
+#pragma unroll
+      for (int u = 0; u < 8; ++u) {
+        const size_t e = (size_t)min(kc + u, c1 - 1) * a.np2 + p;
+        ah[u] = a.th[e];
+        al[u] = a.tl[e];
+      }
+#pragma unroll
+      for (int u = 0; u < 8; ++u) {
+        const int k = kc + u;
+        if (k >= c1) break;
+        const float xv = h == 0 ? xs[j * K + k] : newrow[j * a.rows + (k - c0)];
+        const f2p x2 = pack2(xv, xv);
+        if (k >= a.Kz && k < K) c = pfma(ah[u], x2, c);
+        else pmac(s, c, ah[u], ah[u] ^ 0x8000000080000000ull, al[u], x2);
+      }
+    }
+    float s0, s1, e0, e1;
+    unpack2(s, s0, s1);
+    unpack2(c, e0, e1);
+    const int i0 = (p & 15) + 32 * (p >> 4);
+    float2* dst = a.part + (((size_t)j * gridDim.x + blockIdx.x) * 2 + h) * 2 * a.np2;
+    dst[i0] = make_float2(s0, e0);
+    dst[i0 + 16] = make_float2(s1, e1);
+  }
+}
+
+// new row += U d, d the sum of the Z shares of a job in a fixed order: a warp
+// takes every 32nd share of the R modes, coalesced and all in flight; then a
+// warp a mode adds the 32 sums by a fixed butterfly.
+template <int R>
+__global__ void __launch_bounds__(1024)
+k_step_anchor(int W, int cap, int Z, const StepJobs jobs, const float2* __restrict__ part,
+              const float* __restrict__ u, float* __restrict__ buf) {
+  __shared__ float2 sum[32][R + 1];
+  __shared__ float ds[R];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int j = blockIdx.y, w = blockIdx.x * 1024 + tid;
+  const float2* pj = part + (size_t)j * Z * R;
+#pragma unroll
+  for (int b = 0; b < R; b += 32) {
+    float s = 0.f, c = 0.f;
+#pragma unroll 10
+    for (int z = warp; z < Z; z += 32) {
+      const float2 q = pj[(size_t)z * R + b + lane];
+      c = __fadd_rn(c, q.y);
+      two_sum_acc(s, c, q.x);
+    }
+    sum[warp][b + lane] = make_float2(s, c);
+  }
+  __syncthreads();
+#pragma unroll
+  for (int i = warp; i < R; i += 32) {
+    float s = sum[lane][i].x, c = sum[lane][i].y;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      const float so = __shfl_xor_sync(0xffffffffu, s, o);
+      const float co = __shfl_xor_sync(0xffffffffu, c, o);
+      // the same operands in the same order on both lanes of a pair
+      float s2 = (lane & o) ? so : s, c2 = (lane & o) ? __fadd_rn(co, c) : __fadd_rn(c, co);
+      two_sum_acc(s2, c2, (lane & o) ? s : so);
+      s = s2;
+      c = c2;
+    }
+    if (lane == 0) ds[i] = s + c;
+  }
+  __syncthreads();
+  if (w >= W) return;
+  float v = 0.f;
+#pragma unroll
+  for (int i = 0; i < R; ++i) v = fmaf(__ldg(u + (size_t)i * W + w), ds[i], v);
+  buf[((size_t)jobs.screen[j] * cap + jobs.head[j]) * W + w] += v;
+}
+
+// CTAs of a row step: one per SM, or fewer
+constexpr int kStepCtas = 152;
+constexpr int kStepSmem = 210 * 1024;
+static int step_rows(int W) { return (W + kStepCtas - 1) / kStepCtas; }
+static size_t step_smem(int W, int K, int J) {
+  return ((size_t)J * K + (size_t)J * step_rows(W)) * sizeof(float);
+}
+// A row step of at most kStepJobs plain (rows-only, float32) jobs whose operand
+// fits beside the reduction scratch in shared memory.
+static bool step_fits(int W, int K, int J) {
+  return J <= kStepJobs && step_smem(W, K, J) <= kStepSmem;
+}
+static size_t step_share_bytes(int W, int J, int modes) {
+  const int ctas = (W + step_rows(W) - 1) / step_rows(W);
+  return (size_t)J * 2 * ctas * modes * sizeof(float2);
+}
+
+template <int RT, int JT>
+static int launch_step(const StepArgs& a, const StepJobs& jobs, const StepJobs& next, cudaStream_t s) {
+  const size_t smem = step_smem(a.W, a.K, jobs.n);
+  // the shared-memory limit is a property of the kernel on a device: set once on each
+  static std::atomic<uint64_t> ready{0};
+  int dev = 0;
+  if (int rc = check_cuda(cudaGetDevice(&dev), "k_row_step")) return rc;
+  const uint64_t bit = 1ull << (dev & 63);
+  if (dev > 63 || !(ready.load(std::memory_order_relaxed) & bit)) {
+    if (int rc = check_cuda(cudaFuncSetAttribute(k_row_step<RT, JT>,
+                                                 cudaFuncAttributeMaxDynamicSharedMemorySize, kStepSmem),
+                            "k_row_step"))
+      return rc;
+    if (dev <= 63) ready.fetch_or(bit, std::memory_order_relaxed);
+  }
+  k_row_step<RT, JT><<<(a.W + a.rows - 1) / a.rows, kStepThreads, smem, s>>>(a, jobs, next);
+  return PT_OK;
+}
+template <int RT>
+static int launch_step_j(const StepArgs& a, const StepJobs& jobs, const StepJobs& next, cudaStream_t s) {
+  if (jobs.n <= 1) return launch_step<RT, 1>(a, jobs, next, s);
+  if (jobs.n <= 3) return launch_step<RT, 3>(a, jobs, next, s);
+  if (jobs.n <= 6) return launch_step<RT, 6>(a, jobs, next, s);
+  if (jobs.n <= 9) return launch_step<RT, 9>(a, jobs, next, s);
+  return launch_step<RT, 16>(a, jobs, next, s);
+}
+
 // ---------------------------------------------------------------- readout
 struct RLayer {
   int screen, row_max, anchor_phys;
@@ -650,18 +940,26 @@ __device__ __forceinline__ void taps(float t, float* w) {
   }
 }
 
+// A warp samples an 8 x 4 pixel tile (a CTA 32 x 8): the rotated footprint of a
+// compact tile meets about nine ring rows, where a row of 32 pixels meets up to
+// 32, and each row is a cache line a load has to visit. Where every tap of a
+// tile lies inside the readable rows, the columns and one unbroken stretch of
+// the ring, the taps are fixed offsets from one address a row; the other tiles
+// clamp each tap. 9 layers, cubic, 512^2: 29.0 us with rows of 32 pixels and
+// every tap clamped, 18.9 us so.
 template <int T>
 __global__ void __launch_bounds__(256)
-k_readout(int n, int W, int cap, int L, RLayers P, const float* __restrict__ buf, float scale,
-          float* __restrict__ out) {
-  const int y = blockIdx.x * blockDim.x + threadIdx.x;
-  const int x = blockIdx.y;
-  if (y >= n) return;
-  const int off0 = (T == 2) ? 0 : (T == 4 ? -1 : -2);
+k_readout(int n, int W, int cap, int L, const __grid_constant__ RLayers P,
+          const float* __restrict__ buf, float scale, float* __restrict__ out) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int yt = blockIdx.x * 32 + (warp & 3) * 8 + (lane & 7);
+  const int xt = blockIdx.y * 8 + (warp >> 2) * 4 + (lane >> 3);
+  const int y = min(yt, n - 1), x = min(xt, n - 1);  // lanes outside repeat the edge
+  constexpr int off0 = (T == 2) ? 0 : (T == 4 ? -1 : -2);
   const long long kx = 2ll * x - (n - 1), ky = 2ll * y - (n - 1);
   float acc = 0.f;
   for (int l = 0; l < L; ++l) {
-    const RLayer p = P.l[l];
+    const RLayer& p = P.l[l];
     const long long rowf = kx * p.ca + ky * p.sa + p.ra;
     const long long colf = -kx * p.sa + ky * p.ca + p.rp;
     int r0, c0;
@@ -672,24 +970,47 @@ k_readout(int n, int W, int cap, int L, RLayers P, const float* __restrict__ buf
     taps<T>(fr, wr);
     taps<T>(fc, wc);
     const float* slab = buf + (size_t)p.screen * cap * W;
-    int cc[T];
-#pragma unroll
-    for (int b = 0; b < T; ++b) cc[b] = min(max(c0 + off0 + b, 0), W - 1);
+    r0 += off0;
+    c0 += off0;
+    int phys = p.anchor_phys + r0;
+    if (phys >= cap) phys -= cap;
+    const bool in = r0 >= 0 && r0 + T - 1 <= p.row_max && c0 >= 0 && c0 + T <= W && phys + T <= cap;
     float val = 0.f;
+    if (__all_sync(0xffffffffu, in)) {
+      const float* row = slab + (size_t)phys * W + c0;
+      float v[T][T];
 #pragma unroll
-    for (int a = 0; a < T; ++a) {
-      int rr = min(max(r0 + off0 + a, 0), p.row_max);
-      int phys = p.anchor_phys + rr;
-      if (phys >= cap) phys -= cap;
-      const float* row = slab + (size_t)phys * W;
-      float rs = 0.f;
+      for (int a = 0; a < T; ++a) {
 #pragma unroll
-      for (int b = 0; b < T; ++b) rs = fmaf(wc[b], __ldg(row + cc[b]), rs);
-      val = fmaf(wr[a], rs, val);
+        for (int b = 0; b < T; ++b) v[a][b] = __ldg(row + b);
+        row += W;
+      }
+#pragma unroll
+      for (int a = 0; a < T; ++a) {
+        float rs = 0.f;
+#pragma unroll
+        for (int b = 0; b < T; ++b) rs = fmaf(wc[b], v[a][b], rs);
+        val = fmaf(wr[a], rs, val);
+      }
+    } else {
+      int cc[T];
+#pragma unroll
+      for (int b = 0; b < T; ++b) cc[b] = min(max(c0 + b, 0), W - 1);
+#pragma unroll
+      for (int a = 0; a < T; ++a) {
+        const int rr = min(max(r0 + a, 0), p.row_max);
+        int ph = p.anchor_phys + rr;
+        if (ph >= cap) ph -= cap;
+        const float* row = slab + (size_t)ph * W;
+        float rs = 0.f;
+#pragma unroll
+        for (int b = 0; b < T; ++b) rs = fmaf(wc[b], __ldg(row + cc[b]), rs);
+        val = fmaf(wr[a], rs, val);
+      }
     }
     acc += val;
   }
-  out[(size_t)x * n + y] = scale * acc;
+  if (yt < n && xt < n) out[(size_t)xt * n + yt] = scale * acc;
 }
 
 template <int T>
@@ -816,6 +1137,88 @@ struct ExtrudeForm {
   int incr;                // the operator is in increment form
 };
 
+// Row steps of few screens: one k_row_step (and k_step_anchor) for the jobs of
+// each (step, group), in the workspace [noise (2, J, W) in the operand's place |
+// ... | shares in the partials' place].
+static int step_jobs(const char* who, const ExtrudeForm& form, int W, int m, int cap, float* buf,
+                     int n_jobs, const pt_extrude_job* jobs, const float* noise, void* work,
+                     cudaStream_t s) {
+  const int K = (m + 1) * W;
+  std::vector<std::pair<int, StepJobs>> launches;  // (group, jobs)
+  for (int i = 0; i < n_jobs;) {
+    int e = i;
+    std::map<int, StepJobs> by_group;
+    for (; e < n_jobs && jobs[e].step == jobs[i].step; ++e) {
+      StepJobs& q = by_group[jobs[e].group];
+      const int k = q.n++;
+      q.screen[k] = jobs[e].screen;
+      q.head[k] = jobs[e].head;
+      q.bscale[k] = jobs[e].bscale;
+      q.key[k] = jobs[e].key;
+      q.row[k] = jobs[e].row;
+      q.noise_off[k] = (long long)jobs[e].noise_off;
+    }
+    for (auto& kv : by_group) launches.emplace_back(kv.first, kv.second);
+    i = e;
+  }
+  int max_j = 0;
+  for (auto& q : launches) max_j = std::max(max_j, q.second.n);
+  const Fp32Work fw = fp32_work(W, m, 0, max_j);
+  float* nbuf[2] = {(float*)work, (float*)work + (size_t)max_j * W};
+  const int R = form.anchor ? form.anchor->modes : 0;
+  StepArgs a{};
+  a.W = W;
+  a.m = m;
+  a.cap = cap;
+  a.K = K;
+  a.Kz = m * W;
+  a.rows = step_rows(W);
+  const int ctas = (W + a.rows - 1) / a.rows;
+  a.buf = buf;
+  a.inject = noise;
+  a.np2 = R / 2;
+  a.kslice = (K + ctas - 1) / ctas;
+  a.part = (float2*)((char*)work + fw.x + fw.lo_tiles);
+  {
+    const int pairs = launches[0].second.n * ((W + 1) / 2);
+    k_step_noise<<<(pairs + 255) / 256, 256, 0, s>>>(launches[0].second, W, noise, nbuf[0]);
+    count_launch_e();
+  }
+  const StepJobs none{};
+  for (size_t i = 0; i < launches.size(); ++i) {
+    const int g = launches[i].first;
+    const StepJobs& cur = launches[i].second;
+    a.M = form.M + (size_t)g * W * K;
+    a.noise = nbuf[i & 1];
+    a.noise_next = nbuf[(i + 1) & 1];
+    if (R) {
+      a.th = (const f2p*)form.anchor->t_hi + (size_t)g * (K + W) * a.np2;
+      a.tl = (const f2p*)form.anchor->t_lo + (size_t)g * (K + W) * a.np2;
+    }
+    const StepJobs& nxt = i + 1 < launches.size() ? launches[i + 1].second : none;
+    {
+      ProfScope ps("k_row_step", s);
+      int rc;
+      if (a.rows <= 2) rc = launch_step_j<2>(a, cur, nxt, s);
+      else if (a.rows == 3) rc = launch_step_j<3>(a, cur, nxt, s);
+      else rc = launch_step_j<5>(a, cur, nxt, s);
+      if (rc) return rc;
+    }
+    count_launch_e();
+    if (R) {
+      ProfScope ps("k_step_anchor", s);
+      const dim3 grid((W + 1023) / 1024, cur.n);
+      if (R == 32)
+        k_step_anchor<32><<<grid, 1024, 0, s>>>(W, cap, 2 * ctas, cur, a.part, form.anchor->u, buf);
+      else
+        k_step_anchor<64><<<grid, 1024, 0, s>>>(W, cap, 2 * ctas, cur, a.part, form.anchor->u, buf);
+      count_launch_e();
+    }
+    if (int rc = check_launch(who)) return rc;
+  }
+  return PT_OK;
+}
+
 static int extrude_jobs(const char* who, const ExtrudeForm& form, int W, int m,
                         const pt_sparse_stencil* sparse, int cap, int G, float* buf, int n_jobs,
                         const pt_extrude_job* jobs, const float* noise, void* work,
@@ -851,6 +1254,9 @@ static int extrude_jobs(const char* who, const ExtrudeForm& form, int W, int m,
                                  : pt_extrude_workspace_bytes(W, m, sp.n, max_j);
   if (!work || work_bytes < need) return fail(PT_ERR_ARG, std::string(who) + ": workspace too small");
   const int K = (m + 1) * W + sp.n, Kz = m * W + sp.n;
+  if (form.terms == 0 && !form.lo && !form.incr && sp.n == 0 && step_fits(W, K, max_j) &&
+      step_share_bytes(W, max_j, form.anchor ? form.anchor->modes : 0) <= fp32_work(W, m, 0, max_j).partial)
+    return step_jobs(who, form, W, m, cap, buf, n_jobs, jobs, noise, work, s);
   const int per_launch = form.terms ? tc_max_jobs(form.terms) : kJobsPerLaunch;
   const int jcap = std::min(max_j, per_launch);
   // FP32: X (jcap, K), correction B tiles, partials; tensor cores: B tiles then partials
@@ -1278,7 +1684,7 @@ extern "C" int pt_readout(int n, int W, int cap, int interp, int L, const pt_rea
     P.l[l].rp = std::llround((W / 2.0 + q.shift_perp) * one);
   }
   cudaStream_t s = (cudaStream_t)stream;
-  dim3 grid((n + 255) / 256, n);
+  dim3 grid((n + 31) / 32, (n + 7) / 8);
   ProfScope ps("k_readout", s);
   if (interp == 0) k_readout<2><<<grid, 256, 0, s>>>(n, W, cap, L, P, buf, scale, out);
   else if (interp == 1) k_readout<4><<<grid, 256, 0, s>>>(n, W, cap, L, P, buf, scale, out);
