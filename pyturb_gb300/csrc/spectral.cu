@@ -611,25 +611,26 @@ struct FramePrepArgs {
   double df;
 };
 
-// One CTA per frame, one thread per (level, 3x3 cell): the per-layer phases
-// f_p . s are FP64 products reduced mod 1 (so the error does not grow with the
-// travel), the phasors and the layer sum are float32 (the reference's own
-// complex64 path), and the CTA reduces the grid mean of the low-order screen.
-__global__ void k_frame_coef(FramePrepArgs a, ShiftParams sp, int fbeg, int nf) {
+// Subharmonic coefficients of chunk frame f and their grid mean, by one CTA: a
+// thread per (level, 3x3 cell). The per-layer phases f_p . s are FP64 products
+// reduced mod 1 (so the error does not grow with the travel), the phasors and
+// the layer sum are float32 (the reference's own complex64 path), and the CTA
+// reduces the grid mean of the low-order screen. shift(j, sx, sy) gives the
+// displacement of term j. Every thread of the CTA calls it.
+template <class Shift>
+__device__ __forceinline__ void frame_coef(const FramePrepArgs& a, int f, const Shift& shift) {
   __shared__ double part[32];
-  const int fl = blockIdx.x;
-  if (fl >= nf) return;
-  const int f = fbeg + fl;
   const int t = threadIdx.x;
   double term = 0.0;
-  if (t < a.P * 9) {
-    const int p = t / 9, ij = t % 9, i = ij / 3, k = ij % 3;
+  for (int q = t; q < a.P * 9; q += blockDim.x) {
+    const int p = q / 9, ij = q % 9, i = ij / 3, k = ij % 3;
     const double fi = a.sh_freq[p * 3 + i], fk = a.sh_freq[p * 3 + k];
     float2 acc = make_float2(0.f, 0.f);
+#pragma unroll 3
     for (int j = 0; j < a.J; ++j) {
       const int l = a.per_layer ? a.frame0 + f : j;
-      const double sx = sp.v[(fl * a.J + j) * 2];
-      const double sy = sp.v[(fl * a.J + j) * 2 + 1];
+      double sx, sy;
+      shift(j, sx, sy);
       double ph = fi * sx + fk * sy;
       ph -= floor(ph);
       float sn, cs;
@@ -641,7 +642,7 @@ __global__ void k_frame_coef(FramePrepArgs a, ShiftParams sp, int fbeg, int nf) 
     const double bir = a.beta[(p * 3 + i) * 2], bii = a.beta[(p * 3 + i) * 2 + 1];
     const double bkr = a.beta[(p * 3 + k) * 2], bki = a.beta[(p * 3 + k) * 2 + 1];
     const double br = bir * bkr - bii * bki, bi = bir * bki + bii * bkr;
-    term = (double)acc.x * br - (double)acc.y * bi;
+    term += (double)acc.x * br - (double)acc.y * bi;
   }
   for (int o = 16; o > 0; o >>= 1) term += __shfl_down_sync(0xffffffffu, term, o);
   if ((t & 31) == 0) part[t >> 5] = term;
@@ -651,6 +652,15 @@ __global__ void k_frame_coef(FramePrepArgs a, ShiftParams sp, int fbeg, int nf) 
     for (int w = 0; w < (int)(blockDim.x + 31) / 32; ++w) m += part[w];
     a.mean[f] = (float)m;
   }
+}
+
+__global__ void k_frame_coef(FramePrepArgs a, ShiftParams sp, int fbeg, int nf) {
+  const int fl = blockIdx.x;
+  if (fl >= nf) return;
+  frame_coef(a, fbeg + fl, [&](int j, double& sx, double& sy) {
+    sx = sp.v[(fl * a.J + j) * 2];
+    sy = sp.v[(fl * a.J + j) * 2 + 1];
+  });
 }
 
 // px[f][j][k] = exp(2 pi i f_k sx[f][j]), f_k = k' df, phase wrapped exactly
@@ -709,18 +719,30 @@ __global__ void k_fill_sh(int L, int P, const float* __restrict__ sh_amp,
   sh_coef[i] = make_float2(z.x * amp, z.y * amp);
 }
 
-__global__ void k_boil(size_t n_el, float2* __restrict__ s, const float* __restrict__ amplitude,
-                       const float* __restrict__ tau, float dt, const float* __restrict__ noise,
-                       uint64_t seed, uint64_t call, uint64_t idx_base) {
-  const size_t e = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (e >= n_el) return;
-  const float a = expf(-dt / tau[e]);
+// One AR(1) step of both tables: the grid modes, then the subharmonic ones (the
+// last elements, a few hundred) in the same launch.
+struct BoilPart {
+  size_t n;
+  float2* s;
+  const float* amplitude;
+  const float* tau;
+  const float* noise;  // (2, n) or NULL
+  uint64_t idx_base;
+};
+__global__ void __launch_bounds__(256)
+k_boil(BoilPart main, BoilPart sh, float dt, uint64_t seed, uint64_t call) {
+  size_t e = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+  const bool low = e >= main.n;
+  const BoilPart& p = low ? sh : main;
+  if (low) e -= main.n;
+  if (e >= p.n) return;
+  const float a = expf(-dt / p.tau[e]);
   const float b = sqrtf(fmaxf(1.0f - a * a, 0.0f));
-  const float2 z = noise ? make_float2(noise[e], noise[n_el + e])
-                         : philox_cnormal(seed, idx_base + e, call, kDomainBoil);
-  const float amp = amplitude[e];
-  const float2 v = s[e];
-  s[e] = make_float2(fmaf(a, v.x, b * (z.x * amp)), fmaf(a, v.y, b * (z.y * amp)));
+  const float2 z = p.noise ? make_float2(p.noise[e], p.noise[p.n + e])
+                           : philox_cnormal(seed, p.idx_base + e, call, kDomainBoil);
+  const float amp = p.amplitude[e];
+  const float2 v = p.s[e];
+  p.s[e] = make_float2(fmaf(a, v.x, b * (z.x * amp)), fmaf(a, v.y, b * (z.y * amp)));
 }
 
 // ================================================================ LGS zoom
@@ -745,6 +767,143 @@ __global__ void k_lgs_zoom(int L, int ns, int n, int T, const int32_t* __restric
     acc += v;
   }
   out[(size_t)i * n + j] = scale * acc;
+}
+
+// The same zoom by tiles of kZoomRows x kZoomCols output pixels: the taps are
+// separable, so each source row that a tile meets is interpolated along its
+// columns once, into shared memory, and the rows are combined from there: T
+// loads a pixel and layer (plus T rows in kZoomRows) instead of T^2. The cost of
+// a tile is load latency, layer after layer, so kZoomGroups groups of threads
+// take every kZoomGroups-th layer (their sums are added in order at the end),
+// the row taps of all layers are staged first, and a layer's source values are
+// in flight while the one before is combined. A layer whose tile spans more
+// source rows than the buffer (a magnification above one) takes the direct sum.
+// 9 layers, 512^2, T = 4: 41 us by the direct sum a pixel, 43 us by tiles with
+// one group and no prefetch, 13.4 us so.
+constexpr int kZoomRows = 16, kZoomCols = 64, kZoomThreads = 128, kZoomGroups = 3;
+template <int T>
+static size_t zoom_smem(int L) {
+  return (size_t)L * T * kZoomRows * 8 + (size_t)L * 8 +
+         (size_t)kZoomGroups * 2 * (kZoomRows + T) * kZoomCols * sizeof(float);
+}
+template <int T>
+__global__ void __launch_bounds__(kZoomThreads * kZoomGroups)
+k_lgs_zoom_tile(int L, int ns, int n, const int32_t* __restrict__ idx, const float* __restrict__ w,
+                const float* __restrict__ screens, float scale, float* __restrict__ out) {
+  constexpr int SPAN = kZoomRows + T, G = kZoomThreads / kZoomCols, PX = kZoomRows / G;
+  constexpr int NR = (SPAN + G - 1) / G;  // source rows a thread interpolates
+  extern __shared__ float zs[];
+  float* hbuf = zs;                                                  // (groups, 2, SPAN, cols)
+  float* rw = hbuf + kZoomGroups * 2 * SPAN * kZoomCols;             // (L, T, rows)
+  int* ri = (int*)(rw + (size_t)L * T * kZoomRows);                  // (L, T, rows)
+  int* span = ri + (size_t)L * T * kZoomRows;                        // (L, 2) first and last row
+  const int grp = threadIdx.x / kZoomThreads, t = threadIdx.x % kZoomThreads;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int c = t % kZoomCols, g = t / kZoomCols;
+  const int j = blockIdx.x * kZoomCols + c, i0 = blockIdx.y * kZoomRows;
+  const int jc = min(j, n - 1), rows = min(kZoomRows, n - i0);
+  for (int l = warp; l < L; l += kZoomGroups * kZoomThreads / 32) {
+    int lo = ns, hi = -1;
+    for (int q = lane; q < T * kZoomRows; q += 32) {
+      const size_t e = ((size_t)l * T + q / kZoomRows) * n + min(i0 + q % kZoomRows, n - 1);
+      const int v = idx[e];
+      ri[l * T * kZoomRows + q] = v;
+      rw[l * T * kZoomRows + q] = w[e];
+      lo = min(lo, v);
+      hi = max(hi, v);
+    }
+    lo = __reduce_min_sync(0xffffffffu, lo);
+    hi = __reduce_max_sync(0xffffffffu, hi);
+    if (lane == 0) {
+      span[2 * l] = lo;
+      span[2 * l + 1] = hi;
+    }
+  }
+  float acc[PX];
+#pragma unroll
+  for (int q = 0; q < PX; ++q) acc[q] = 0.f;
+  int ci[T];
+  float cw[T], nw[T];
+  float v[NR][T];
+  auto columns = [&](int l) {  // column taps of layer l
+#pragma unroll
+    for (int a = 0; a < T; ++a) {
+      ci[a] = idx[((size_t)l * T + a) * n + jc];
+      nw[a] = w[((size_t)l * T + a) * n + jc];
+    }
+  };
+  auto fetch = [&](int l) {  // this thread's source values of layer l
+    const int lo = span[2 * l], last = min(span[2 * l + 1] - lo, SPAN - 1);
+    const float* s = screens + (size_t)l * ns * ns + (size_t)lo * ns;
+#pragma unroll
+    for (int q = 0; q < NR; ++q) {
+      const float* row = s + (size_t)min(g + q * G, last) * ns;
+#pragma unroll
+      for (int a = 0; a < T; ++a) v[q][a] = __ldg(row + ci[a]);
+    }
+  };
+  if (grp < L) columns(grp);
+  __syncthreads();
+  if (grp < L) fetch(grp);
+  int b = 0;
+  for (int l = grp; l < L; l += kZoomGroups) {
+    float* h = hbuf + (size_t)(grp * 2 + b) * SPAN * kZoomCols;
+    const int lo = span[2 * l];
+    const bool fits = span[2 * l + 1] - lo < SPAN;
+    const int* rl = ri + l * T * kZoomRows;
+    const float* wl = rw + l * T * kZoomRows;
+    if (!fits) {
+#pragma unroll
+      for (int q = 0; q < PX; ++q) {
+        float sum = 0.f;
+        for (int a = 0; a < T; ++a) {
+          const float* row = screens + (size_t)l * ns * ns + (size_t)rl[a * kZoomRows + g + q * G] * ns;
+          float rs = 0.f;
+#pragma unroll
+          for (int k = 0; k < T; ++k) rs = fmaf(nw[k], __ldg(row + ci[k]), rs);
+          sum = fmaf(wl[a * kZoomRows + g + q * G], rs, sum);
+        }
+        acc[q] += sum;
+      }
+    }
+#pragma unroll
+    for (int a = 0; a < T; ++a) cw[a] = nw[a];
+    if (l + kZoomGroups < L) columns(l + kZoomGroups);
+#pragma unroll
+    for (int q = 0; q < NR; ++q) {
+      float rs = 0.f;
+#pragma unroll
+      for (int a = 0; a < T; ++a) rs = fmaf(cw[a], v[q][a], rs);
+      if (g + q * G < SPAN) h[(g + q * G) * kZoomCols + c] = rs;
+    }
+    if (l + kZoomGroups < L) fetch(l + kZoomGroups);
+    // the other buffer was last read before the barrier of the layer before
+    asm volatile("bar.sync %0, %1;" ::"r"(1 + grp), "n"(kZoomThreads) : "memory");
+    if (fits) {
+#pragma unroll
+      for (int q = 0; q < PX; ++q) {
+        float sum = 0.f;
+#pragma unroll
+        for (int a = 0; a < T; ++a)
+          sum = fmaf(wl[a * kZoomRows + g + q * G],
+                     h[(rl[a * kZoomRows + g + q * G] - lo) * kZoomCols + c], sum);
+        acc[q] += sum;
+      }
+    }
+    b ^= 1;
+  }
+  // the groups' sums, in group order (hbuf is free once every group is here)
+  __syncthreads();
+#pragma unroll
+  for (int q = 0; q < PX; ++q) hbuf[(grp * kZoomRows + g + q * G) * kZoomCols + c] = acc[q];
+  __syncthreads();
+  for (int e = threadIdx.x; e < kZoomRows * kZoomCols; e += kZoomThreads * kZoomGroups) {
+    const int r = e / kZoomCols, jj = blockIdx.x * kZoomCols + e % kZoomCols;
+    float s = hbuf[e];
+#pragma unroll
+    for (int q = 1; q < kZoomGroups; ++q) s += hbuf[q * kZoomRows * kZoomCols + e];
+    if (r < rows && jj < n) out[(size_t)(i0 + r) * n + jj] = scale * s;
+  }
 }
 
 #include "frames_fast.cuh"  // power-of-two fast path kernels
@@ -954,6 +1113,54 @@ static int launch_uniform_reg_chunk(const pt_grid* g, const float2* spectra, con
   if (L <= 9) return uniform_reg_rows_t<9>(g, spectra, L, nf, ut, w.hn, w.img, s);
   if (L <= 12) return uniform_reg_rows_t<12>(g, spectra, L, nf, ut, w.hn, w.img, s);
   return uniform_reg_rows_t<16>(g, spectra, L, nf, ut, w.hn, w.img, s);
+}
+
+// ---- frames at arbitrary shifts on power-of-two grids
+static bool frames_reg(int ns, int J) {
+  return ns >= 128 && ns <= 2048 && (ns & (ns - 1)) == 0 && 2 * J <= kShiftTermsMany;
+}
+
+template <int N, int CAP>
+static int frame_rows_reg_t(const pt_grid* g, const float2* spectra, const FramePrepArgs& pa,
+                            const double* sx, const double* sy, int f0, float2* img,
+                            cudaStream_t s) {
+  using Cfg = FrameRowsCfg<N>;
+  const size_t smem = (size_t)(N + 4 * fft_padded(N) + 2 * pa.J) * sizeof(float2);
+  auto kern = k_frame_rows_reg<N, CAP>;
+  if (int rc = set_smem(kern, smem, "k_frame_rows_reg")) return rc;
+  const int fsub = CAP / pa.J & ~1;  // frames a launch takes, whole pairs
+  for (int fb = 0; fb < pa.F; fb += fsub) {
+    const int nf = std::min(fsub, pa.F - fb);
+    FrameShifts<CAP> sh;
+    for (int f = 0; f < nf; ++f)
+      for (int j = 0; j < pa.J; ++j) {
+        const size_t gf = (size_t)f0 + fb + f;
+        const size_t src = pa.per_layer ? gf : gf * pa.J + j;
+        sh.v[f * pa.J + j] = FrameShift{sx[src], sy[src], host_fixed(sx[src] * pa.df),
+                                        host_fixed(sy[src] * pa.df)};
+      }
+    ProfScope ps("k_frame_rows", s);
+    kern<<<dim3(N / 2 + 1 + (pa.P > 0), (nf + 1) / 2), Cfg::THREADS, smem, s>>>(g->tw, spectra, pa,
+                                                                               sh, fb, nf, img);
+    if (fb) count_launch();  // the caller counts one
+  }
+  return PT_OK;
+}
+
+static int launch_frame_rows_reg(const pt_grid* g, const float2* spectra, const FramePrepArgs& pa,
+                                 const double* sx, const double* sy, int f0, float2* img,
+                                 cudaStream_t s) {
+  // a few shifts travel in 2 KB of launch parameters, many in 16 KB
+  const bool few = pa.F * pa.J <= kShiftTermsFew && 2 * pa.J <= kShiftTermsFew;
+  switch (g->ns) {
+#define PT_CASE(n)                                                                             \
+  case n:                                                                                      \
+    return few ? frame_rows_reg_t<n, kShiftTermsFew>(g, spectra, pa, sx, sy, f0, img, s)       \
+               : frame_rows_reg_t<n, kShiftTermsMany>(g, spectra, pa, sx, sy, f0, img, s);
+    PT_CASE(128) PT_CASE(256) PT_CASE(512) PT_CASE(1024) PT_CASE(2048)
+#undef PT_CASE
+  }
+  return fail(PT_ERR_UNSUPPORTED, "frame_rows_reg: not an instantiated size");
 }
 
 // ---- power-of-two dispatch (runtime ns -> template N)
@@ -1607,7 +1814,13 @@ extern "C" int pt_frames(const pt_grid* g, int L, const float* spectra, const fl
                                             sx, sy, f0, nf, w, s))
         return rc;
     }
-    for (int fb = 0; fb < nf && !uni_reg; fb += fsub) {
+    const bool reg = !uni && frames_reg(ns, J);
+    if (reg) {
+      // phasors, layer sums, row transforms and coefficients in one launch
+      if (int rc = launch_frame_rows_reg(g, (const float2*)spectra, pa, sx, sy, f0, w.img, s))
+        return rc;
+    }
+    for (int fb = 0; fb < nf && !uni_reg && !reg; fb += fsub) {
       const int nb = std::min(fsub, nf - fb);
       ShiftParams sp;
       for (int f = 0; f < nb; ++f)
@@ -1626,7 +1839,7 @@ extern "C" int pt_frames(const pt_grid* g, int L, const float* spectra, const fl
       k_frame_phasors<<<dim3((ns + 255) / 256, nb * J), 256, 0, s>>>(pa, sp, fb);
       count_launch();
     }
-    if (uni_reg) {
+    if (uni_reg || reg) {
       // rows done above
     } else if (uni) {
       if (int rc = launch_uniform_rows(g, (const float2*)spectra, L, sx, sy, f0, nf, w.hn, w.px,
@@ -1675,7 +1888,20 @@ extern "C" int pt_lgs_zoom(int L, int ns, int n, int T, const int32_t* idx, cons
   if (L < 1 || ns < 1 || n < 1 || T < 1 || T > 6) return fail(PT_ERR_ARG, "pt_lgs_zoom: bad sizes");
   if (!idx || !w || !screens || !out) return fail(PT_ERR_ARG, "pt_lgs_zoom: NULL pointer");
   cudaStream_t s = (cudaStream_t)stream;
-  k_lgs_zoom<<<dim3((n + 127) / 128, n), 128, 0, s>>>(L, ns, n, T, idx, w, screens, scale, out);
+  ProfScope ps("k_lgs_zoom", s);
+  const dim3 tiles((n + kZoomCols - 1) / kZoomCols, (n + kZoomRows - 1) / kZoomRows);
+  auto go = [&](auto kern, size_t smem) -> int {
+    if (int rc = set_smem(kern, smem, "k_lgs_zoom_tile")) return rc;
+    kern<<<tiles, kZoomThreads * kZoomGroups, smem, s>>>(L, ns, n, idx, w, screens, scale, out);
+    return PT_OK;
+  };
+  // the staged row taps of up to 150 layers fit beside the tiles
+  int rc = PT_OK;
+  if (T == 2 && L <= 150) rc = go(k_lgs_zoom_tile<2>, zoom_smem<2>(L));
+  else if (T == 4 && L <= 150) rc = go(k_lgs_zoom_tile<4>, zoom_smem<4>(L));
+  else if (T == 6 && L <= 150) rc = go(k_lgs_zoom_tile<6>, zoom_smem<6>(L));
+  else k_lgs_zoom<<<dim3((n + 127) / 128, n), 128, 0, s>>>(L, ns, n, T, idx, w, screens, scale, out);
+  if (rc) return rc;
   count_launch();
   return check_launch("pt_lgs_zoom");
 }
@@ -1689,17 +1915,11 @@ extern "C" int pt_boil_step(const pt_grid* g, int L, float* spectra, float* sh_c
   if (g->P > 0 && (!sh_coef || !sh_amp || !sh_tau)) return fail(PT_ERR_ARG, "pt_boil_step: NULL subharmonic table");
   if (!(dt > 0)) return fail(PT_ERR_ARG, "pt_boil_step: dt must be positive");
   cudaStream_t s = (cudaStream_t)stream;
-  const size_t n_main = (size_t)L * g->ns * g->ns;
-  k_boil<<<(unsigned)((n_main + 255) / 256), 256, 0, s>>>(n_main, (float2*)spectra, amplitude,
-                                                         main_tau, (float)dt, noise, seed, call, 0);
+  const size_t n_main = (size_t)L * g->ns * g->ns, n_sh = (size_t)g->P * L * 9;
+  const BoilPart mp{n_main, (float2*)spectra, amplitude, main_tau, noise, 0};
+  const BoilPart sp{n_sh, (float2*)sh_coef, sh_amp, sh_tau, sh_noise, 1ull << 40};
+  k_boil<<<(unsigned)((n_main + n_sh + 255) / 256), 256, 0, s>>>(mp, sp, (float)dt, seed, call);
   count_launch();
-  if (g->P > 0) {
-    const size_t n_sh = (size_t)g->P * L * 9;
-    k_boil<<<(unsigned)((n_sh + 127) / 128), 128, 0, s>>>(n_sh, (float2*)sh_coef, sh_amp, sh_tau,
-                                                         (float)dt, sh_noise, seed, call,
-                                                         1ull << 40);
-    count_launch();
-  }
   return check_launch("pt_boil_step");
 }
 
