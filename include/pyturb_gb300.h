@@ -474,7 +474,12 @@ int pt_tc_probe(int N, int K, const uint16_t* A, const uint16_t* B, float* D, vo
  *     (F, 18 P + 1) f64 = per frame the projections sum_xy g_f(x, y)
  *     b_pi(crop + x) b_pj(crop + y) (re, im; p, i, j row-major) on the grid's
  *     basis rows b_pi(x) = exp(2 pi i f_pi (x - ns/2) dx), then sum_xy g_f;
- *     the caller forms the level gradients from these (9 P values a frame). */
+ *  7. pt_synth_adj_levels: the chunk's frames [f0, f0 + F) folded into
+ *     grad_w (L) f64, grad_shifts (all frames, L, 2) f64 (both or neither) and
+ *     grad_coef (L, P, 3, 3) complex f64 (d/dRe + i d/dIm; may be NULL) from
+ *     out of step 5 (`part`, may be NULL) and step 6 (`proj`, may be NULL; then
+ *     sh_coef (P, L, 3, 3) complex and the DEVICE shifts of the chunk are
+ *     needed). grad_w and grad_coef are added to when accumulate != 0. */
 int pt_synth_adj_pack(int ns, int F, int crop, int n_out, float scale, const float* g, float* z,
                       void* stream);
 int pt_synth_adj_phasors(int ns, double pixel_scale, int L, int F, const double* sx,
@@ -486,6 +491,12 @@ int pt_synth_adj_params(int ns, double pixel_scale, int L, int F, const float* w
                         void* stream);
 int pt_synth_adj_sh(const pt_grid* grid, int F, int crop, int n_out, const float* g, double* out,
                     void* stream);
+size_t pt_synth_adj_levels_workspace_bytes(int L, int F, int P);
+int pt_synth_adj_levels(const pt_grid* grid, int L, int F, int f0, float scale, const float* w,
+                        const float* sh_coef, const double* sx, const double* sy,
+                        const double* proj, const double* part, int accumulate, double* grad_w,
+                        double* grad_shifts, double* grad_coef, void* work, size_t work_bytes,
+                        void* stream);
 
 #ifdef __cplusplus
 }

@@ -162,6 +162,9 @@ SIGNATURES = {
     "pt_synth_adj_spectra": (i32, [i32, i32, i32, vp, vp, vp, i32, vp, vp]),
     "pt_synth_adj_params": (i32, [i32, f64, i32, i32, vp, vp, vp, vp, vp, vp]),
     "pt_synth_adj_sh": (i32, [vp, i32, i32, i32, vp, vp, vp]),
+    "pt_synth_adj_levels_workspace_bytes": (sz, [i32, i32, i32]),
+    "pt_synth_adj_levels": (i32, [vp, i32, i32, i32, f32, vp, vp, vp, vp, vp, vp, i32, vp, vp, vp,
+                                  vp, sz, vp]),
 }
 
 

@@ -2091,6 +2091,105 @@ __global__ void k_translate_sh(int P, int L, TranslateArgs a, const double* __re
 // crop window, the projections
 //   out[f][((p*3 + i)*3 + j)*2 + {re, im}] = sum_{x,y} g_f(x, y) b_pi(crop + x) b_pj(crop + y)
 //   out[f][18 P] = sum_{x,y} g_f(x, y)
+// Symmetric frequencies (b_1 = 1, b_2 = conj b_0; g is real): a level needs the
+// complex column sums u(y) = sum_x g b_0 and nine real sums over y. One CTA per
+// frame, kShCols columns x kShSlices row slices of threads, float sums along a
+// slice (short runs in flight together) added over the slices, NL levels a pass
+// over g; then kShCols threads a level form the sums over y in FP64, a fixed
+// order throughout. FP64 runs at 1/64 of the FP32 rate here, so its products
+// are what the symmetry leaves. 32 frames of 256^2, 3 levels: 102 us with 256
+// threads walking whole columns, all nine complex products in FP64 and one pass
+// a level (k_adj_sh, still the form for other frequencies), 21.7 us so.
+constexpr int kShCols = 128, kShSlices = 8;
+template <int NL>
+__global__ void __launch_bounds__(kShCols * kShSlices)
+k_adj_sh_sym(int ns, int P, int p0, int crop, int n_out, const float2* __restrict__ basis,
+             const float* __restrict__ g, double* __restrict__ out) {
+  __shared__ float part[kShSlices][2 * NL + 1][kShCols];
+  __shared__ double red[NL][kShCols / 32][9];
+  const int f = blockIdx.x;
+  const float* gf = g + (size_t)f * n_out * n_out;
+  const int c = threadIdx.x % kShCols, sl = threadIdx.x / kShCols;
+  const int rows = (n_out + kShSlices - 1) / kShSlices;
+  const int xb = min(n_out, sl * rows), xe = min(n_out, xb + rows);
+  const float2* bp = basis + (size_t)p0 * 3 * ns + crop;  // row 0 of each level
+  double acc[9];
+#pragma unroll
+  for (int q = 0; q < 9; ++q) acc[q] = 0.0;
+  for (int y0 = 0; y0 < n_out; y0 += kShCols) {
+    const int y = y0 + c;
+    float2 u[NL];
+    float sum = 0.f;
+#pragma unroll
+    for (int l = 0; l < NL; ++l) u[l] = make_float2(0.f, 0.f);
+    if (y < n_out) {
+#pragma unroll 8
+      for (int x = xb; x < xe; ++x) {
+        const float v = __ldg(gf + (size_t)x * n_out + y);
+        sum += v;
+#pragma unroll
+        for (int l = 0; l < NL; ++l) {
+          const float2 b = __ldg(bp + (size_t)(3 * l) * ns + x);
+          u[l].x = fmaf(b.x, v, u[l].x);
+          u[l].y = fmaf(b.y, v, u[l].y);
+        }
+      }
+    }
+    part[sl][0][c] = sum;
+#pragma unroll
+    for (int l = 0; l < NL; ++l) {
+      part[sl][1 + 2 * l][c] = u[l].x;
+      part[sl][2 + 2 * l][c] = u[l].y;
+    }
+    __syncthreads();
+    if (sl < NL && y < n_out) {  // threads of slice l sum level l
+      float t = 0.f, ux = 0.f, uy = 0.f;
+#pragma unroll
+      for (int q = 0; q < kShSlices; ++q) {
+        t += part[q][0][c];
+        ux += part[q][1 + 2 * sl][c];
+        uy += part[q][2 + 2 * sl][c];
+      }
+      const float2 b = __ldg(bp + (size_t)(3 * sl) * ns + y);
+      const double dx = ux, dy = uy, dt = t, bx = b.x, by = b.y;
+      acc[0] += dx * bx;
+      acc[1] += dy * by;
+      acc[2] += dx * by;
+      acc[3] += dy * bx;
+      acc[4] += dx;
+      acc[5] += dy;
+      acc[6] += dt * bx;
+      acc[7] += dt * by;
+      acc[8] += dt;
+    }
+    __syncthreads();
+  }
+  if (sl >= NL) return;
+#pragma unroll
+  for (int q = 0; q < 9; ++q) {
+    double v = acc[q];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    if ((c & 31) == 0) red[sl][c >> 5][q] = v;
+  }
+  asm volatile("bar.sync %0, %1;" ::"r"(1 + sl), "n"(kShCols) : "memory");
+  if (c != 0) return;
+  double v[9];
+#pragma unroll
+  for (int q = 0; q < 9; ++q) {
+    v[q] = 0.0;
+#pragma unroll
+    for (int w = 0; w < kShCols / 32; ++w) v[q] += red[sl][w][q];
+  }
+  const double G[18] = {v[0] - v[1], v[2] + v[3], v[4],  v[5],  v[0] + v[1], v[3] - v[2],
+                        v[6],        v[7],        v[8],  0.0,   v[6],        -v[7],
+                        v[0] + v[1], v[2] - v[3], v[4],  -v[5], v[0] - v[1], -(v[2] + v[3])};
+  double* of = out + (size_t)f * (18 * P + 1);
+#pragma unroll
+  for (int q = 0; q < 18; ++q) of[(size_t)(p0 + sl) * 18 + q] = G[q];
+  if (p0 + sl == 0) of[(size_t)18 * P] = v[8];
+}
+
 // One CTA per frame; thread t owns columns y = t, t + 256, ...; one pass over
 // g per level; float sums along x, double products and a fixed-order reduce.
 __global__ void __launch_bounds__(256)
@@ -2149,6 +2248,147 @@ k_adj_sh(int ns, int P, int crop, int n_out, const float2* __restrict__ basis,
   }
 }
 
+// Level gradients from the projections. With C_fpij = sum_l w_l c_lpij E_flpij,
+// E = exp(2 pi i (sx f_pi + sy f_pj)) and Q = scale (G - beta_pi beta_pj sum g),
+//   dL/dw_l += sum Re(c E Q), dL/dsx_fl -= 2 pi sum f_pi Im(w c E Q) (sy: f_pj),
+//   dL/dc_lpij += conj(w_l sum_f E Q),
+// in FP64. k_adj_terms: CTA = (frame, layer), thread = (p, i, j); it writes
+// E Q and the frame's shift gradient (with the grid part's, if given).
+// k_adj_levels: CTA = layer, sums over the frames in order.
+struct AdjLevels {
+  int L, F, P, f0;        // F frames of this chunk, the first is frame f0
+  double scale;
+  const double* freq;     // (P, 3)
+  const double* beta;     // (P, 3, 2)
+  const float* w;         // (L)
+  const float2* c;        // (P, L, 9)
+  const double* sx;       // (F, L)
+  const double* sy;
+  const double* proj;     // (F, 18 P + 1), or NULL: no levels
+  const double* part;     // (L, F, 3) of pt_synth_adj_params, or NULL
+  double2* eq;            // (F, L, 9 P)
+  double* fw;             // (F, L) weight contributions
+  double* gw;             // (L)
+  double* gsh;            // (all frames, L, 2)
+  double2* gc;            // (L, P, 9), or NULL
+  int accumulate;
+};
+
+__global__ void __launch_bounds__(160)
+k_adj_terms(AdjLevels a) {
+  __shared__ double red[5][3];
+  const int f = blockIdx.x, l = blockIdx.y, t = threadIdx.x;
+  double v[3] = {0.0, 0.0, 0.0};
+  if (a.proj && t < 9 * a.P) {
+    const int p = t / 9, ij = t % 9, i = ij / 3, j = ij % 3;
+    const double* pr = a.proj + (size_t)f * (18 * a.P + 1);
+    const double fi = a.freq[3 * p + i], fj = a.freq[3 * p + j];
+    const double bir = a.beta[(3 * p + i) * 2], bii = a.beta[(3 * p + i) * 2 + 1];
+    const double bjr = a.beta[(3 * p + j) * 2], bji = a.beta[(3 * p + j) * 2 + 1];
+    const double S = pr[18 * a.P];
+    const double qr = a.scale * (pr[2 * t] - (bir * bjr - bii * bji) * S);
+    const double qi = a.scale * (pr[2 * t + 1] - (bir * bji + bii * bjr) * S);
+    double ph = a.sx[(size_t)f * a.L + l] * fi + a.sy[(size_t)f * a.L + l] * fj;
+    ph -= floor(ph);
+    double sn, cs;
+    sincospi(2.0 * ph, &sn, &cs);
+    const double er = cs * qr - sn * qi, ei = cs * qi + sn * qr;
+    a.eq[((size_t)f * a.L + l) * 9 * a.P + t] = make_double2(er, ei);
+    const float2 c = a.c[((size_t)p * a.L + l) * 9 + ij];
+    v[0] = (double)c.x * er - (double)c.y * ei;
+    const double im = (double)a.w[l] * ((double)c.x * ei + (double)c.y * er);
+    v[1] = fi * im;
+    v[2] = fj * im;
+  }
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v[k] += __shfl_xor_sync(0xffffffffu, v[k], o);
+    if ((t & 31) == 0) red[t >> 5][k] = v[k];
+  }
+  __syncthreads();
+  if (t < 3) {
+    double s = 0.0;
+    for (int q = 0; q < (int)(blockDim.x >> 5); ++q) s += red[q][t];
+    const double grid = a.part ? a.part[((size_t)l * a.F + f) * 3 + t] : 0.0;
+    if (t == 0) a.fw[(size_t)f * a.L + l] = s + grid;
+    else if (a.gsh) a.gsh[((size_t)(a.f0 + f) * a.L + l) * 2 + t - 1] = grid - 2.0 * M_PI * s;
+  }
+}
+
+__global__ void __launch_bounds__(160)
+k_adj_levels(AdjLevels a) {
+  const int l = blockIdx.x, t = threadIdx.x;
+  const int Q = a.proj && a.gc ? 9 * a.P : 0;
+  if (t < Q) {
+    double2 s = make_double2(0.0, 0.0);
+#pragma unroll 8
+    for (int f = 0; f < a.F; ++f) {
+      const double2 v = a.eq[((size_t)f * a.L + l) * 9 * a.P + t];
+      s.x += v.x;
+      s.y += v.y;
+    }
+    double2* o = a.gc + (size_t)l * Q + t;
+    const double w = a.w[l];
+    const double2 was = a.accumulate ? *o : make_double2(0.0, 0.0);
+    *o = make_double2(was.x + w * s.x, was.y - w * s.y);
+  }
+  if (t == 159 && a.gw) {
+    double s = a.accumulate ? a.gw[l] : 0.0;
+#pragma unroll 8
+    for (int f = 0; f < a.F; ++f) s += a.fw[(size_t)f * a.L + l];
+    a.gw[l] = s;
+  }
+}
+
+extern "C" size_t pt_synth_adj_levels_workspace_bytes(int L, int F, int P) {
+  if (L < 1 || F < 1 || P < 0 || P > kMaxLevels) return 0;
+  return ((size_t)18 * P + 1) * L * F * sizeof(double);
+}
+
+extern "C" int pt_synth_adj_levels(const pt_grid* g, int L, int F, int f0, float scale, const float* w,
+                                   const float* sh_coef, const double* sx, const double* sy,
+                                   const double* proj, const double* part, int accumulate,
+                                   double* grad_w, double* grad_shifts, double* grad_coef, void* work,
+                                   size_t work_bytes, void* stream) {
+  if (int rc = check_grid(g, "pt_synth_adj_levels")) return rc;
+  if (L < 1 || L > 65535 || F < 1 || f0 < 0) return fail(PT_ERR_ARG, "pt_synth_adj_levels: bad sizes");
+  if (!w || (!proj && !part) || (!grad_w != !grad_shifts))
+    return fail(PT_ERR_ARG, "pt_synth_adj_levels: NULL pointer");
+  if (proj && (g->P < 1 || !sh_coef || !sx || !sy))
+    return fail(PT_ERR_ARG, "pt_synth_adj_levels: projections without levels, coefficients or shifts");
+  if (grad_coef && !proj) return fail(PT_ERR_ARG, "pt_synth_adj_levels: level gradients need projections");
+  const int P = proj ? g->P : 0;
+  if (!work || work_bytes < pt_synth_adj_levels_workspace_bytes(L, F, P))
+    return fail(PT_ERR_ARG, "pt_synth_adj_levels: workspace too small");
+  AdjLevels a{};
+  a.L = L;
+  a.F = F;
+  a.P = P;
+  a.f0 = f0;
+  a.scale = scale;
+  a.freq = g->sh_freq;
+  a.beta = g->beta;
+  a.w = w;
+  a.c = (const float2*)sh_coef;
+  a.sx = sx;
+  a.sy = sy;
+  a.proj = proj;
+  a.part = part;
+  a.eq = (double2*)work;
+  a.fw = (double*)work + (size_t)18 * P * L * F;
+  a.gw = grad_w;
+  a.gsh = grad_shifts;
+  a.gc = (double2*)grad_coef;
+  a.accumulate = accumulate;
+  cudaStream_t s = (cudaStream_t)stream;
+  ProfScope ps("k_adj_levels", s);
+  k_adj_terms<<<dim3(F, L), 32 * std::max(1, (9 * P + 31) / 32), 0, s>>>(a);
+  k_adj_levels<<<L, 160, 0, s>>>(a);
+  count_launch(2);
+  return check_launch("pt_synth_adj_levels");
+}
+
 extern "C" int pt_synth_adj_sh(const pt_grid* g, int F, int crop, int n_out, const float* grad,
                                double* out, void* stream) {
   if (int rc = check_grid(g, "pt_synth_adj_sh")) return rc;
@@ -2158,7 +2398,18 @@ extern "C" int pt_synth_adj_sh(const pt_grid* g, int F, int crop, int n_out, con
   if (!grad || !out) return fail(PT_ERR_ARG, "pt_synth_adj_sh: NULL pointer");
   cudaStream_t s = (cudaStream_t)stream;
   ProfScope ps("k_adj_sh", s);
-  k_adj_sh<<<F, 256, 0, s>>>(g->ns, g->P, crop, n_out, g->basis, grad, out);
+  if (!g->sym) {
+    k_adj_sh<<<F, 256, 0, s>>>(g->ns, g->P, crop, n_out, g->basis, grad, out);
+  } else {
+    for (int p = 0; p < g->P;) {  // up to three levels a pass over the gradient
+      const int nl = std::min(3, g->P - p), threads = kShCols * kShSlices;
+      if (nl == 1) k_adj_sh_sym<1><<<F, threads, 0, s>>>(g->ns, g->P, p, crop, n_out, g->basis, grad, out);
+      else if (nl == 2) k_adj_sh_sym<2><<<F, threads, 0, s>>>(g->ns, g->P, p, crop, n_out, g->basis, grad, out);
+      else k_adj_sh_sym<3><<<F, threads, 0, s>>>(g->ns, g->P, p, crop, n_out, g->basis, grad, out);
+      p += nl;
+      if (p < g->P) count_launch();
+    }
+  }
   count_launch();
   return check_launch("pt_synth_adj_sh");
 }

@@ -105,13 +105,25 @@ __global__ void k_adj_spectra(int ns, int L, int F, const float* __restrict__ w,
   gs[(size_t)l * npix + k] = v;
 }
 
+// s + x into (s, c): s the rounded sum, c collects the rounding errors
+__device__ __forceinline__ void pair_add(float2& a, float x) {
+  const float t = __fadd_rn(a.x, x);
+  const float bv = __fsub_rn(t, a.x);
+  a.y = __fadd_rn(a.y, __fadd_rn(__fsub_rn(a.x, __fsub_rn(t, bv)), __fsub_rn(x, bv)));
+  a.x = t;
+}
+
 // Per (layer, frame pair): [sum Re q, -2 pi w sum fx Im q, -2 pi w sum fy Im q]
-// with q = conj(G_f) S_l Phi_lf, for both frames of the pair, in float64.
-__global__ void __launch_bounds__(256)
+// with q = conj(G_f) S_l Phi_lf, for both frames of the pair, a warp a spectrum
+// row. The sums are kept as float pairs (error-free two-sums) and turned to
+// float64 for the reduction: FP64 adds, at 1/64 of the FP32 rate here, bounded
+// the kernel. 9 layers, 32 frames of 256^2: 258 us with six FP64 adds an
+// element and 256 threads, 53 us so (instruction issue).
+__global__ void __launch_bounds__(1024)
 k_adj_params(int ns, double df, int L, int F, const float* __restrict__ w,
              const float2* __restrict__ spectra, const float2* __restrict__ Z,
              const float2* __restrict__ ph, double* __restrict__ out) {
-  __shared__ double red[8][6];
+  __shared__ double red[32][6];
   const int l = blockIdx.x, p = blockIdx.y;
   const size_t npix = (size_t)ns * ns;
   const float2* S = spectra + (size_t)l * npix;
@@ -119,29 +131,37 @@ k_adj_params(int ns, double df, int L, int F, const float* __restrict__ w,
   const bool two = 2 * p + 1 < F;
   const float2* p0 = ph + ((size_t)l * F + 2 * p) * 2 * ns;
   const float2* p1 = two ? p0 + 2 * ns : p0;
-  double acc[6] = {0, 0, 0, 0, 0, 0};
-  for (size_t k = threadIdx.x; k < npix; k += blockDim.x) {
-    const int kr = (int)(k / ns), kc = (int)(k % ns);
-    const size_t nk = (size_t)((ns - kr) % ns) * ns + (ns - kc) % ns;
-    float2 ga, gb;
-    split_pair(Zp[k], Zp[nk], ga, gb);
-    const float2 s = S[k];
-    const float fxr = (float)signed_freq(kr, ns), fyc = (float)signed_freq(kc, ns);
-    const float2 q0 = cmul(cconj(ga), cmul(s, cmul(p0[kr], p0[ns + kc])));
-    acc[0] += q0.x;
-    acc[1] += fxr * q0.y;
-    acc[2] += fyc * q0.y;
-    if (two) {
-      const float2 q1 = cmul(cconj(gb), cmul(s, cmul(p1[kr], p1[ns + kc])));
-      acc[3] += q1.x;
-      acc[4] += fxr * q1.y;
-      acc[5] += fyc * q1.y;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
+  float2 acc[6];
+#pragma unroll
+  for (int i = 0; i < 6; ++i) acc[i] = make_float2(0.f, 0.f);
+  for (int kr = warp; kr < ns; kr += warps) {
+    const float2* zrow = Zp + (size_t)kr * ns;
+    const float2* nrow = Zp + (size_t)(kr == 0 ? 0 : ns - kr) * ns;
+    const float2* srow = S + (size_t)kr * ns;
+    const float2 x0 = p0[kr], x1 = p1[kr];
+    const float fxr = (float)signed_freq(kr, ns);
+#pragma unroll 4
+    for (int kc = lane; kc < ns; kc += 32) {
+      float2 ga, gb;
+      split_pair(zrow[kc], nrow[kc == 0 ? 0 : ns - kc], ga, gb);
+      const float2 s = srow[kc];
+      const float fyc = (float)signed_freq(kc, ns);
+      const float2 q0 = cmul(cconj(ga), cmul(s, cmul(x0, p0[ns + kc])));
+      pair_add(acc[0], q0.x);
+      pair_add(acc[1], fxr * q0.y);
+      pair_add(acc[2], fyc * q0.y);
+      if (two) {
+        const float2 q1 = cmul(cconj(gb), cmul(s, cmul(x1, p1[ns + kc])));
+        pair_add(acc[3], q1.x);
+        pair_add(acc[4], fxr * q1.y);
+        pair_add(acc[5], fyc * q1.y);
+      }
     }
   }
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 #pragma unroll
   for (int i = 0; i < 6; ++i) {
-    double v = acc[i];
+    double v = (double)acc[i].x + (double)acc[i].y;
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
     if (lane == 0) red[warp][i] = v;
@@ -150,7 +170,7 @@ k_adj_params(int ns, double df, int L, int F, const float* __restrict__ w,
   if (threadIdx.x < 6) {
     const int i = threadIdx.x;
     double v = 0.0;
-    for (int q = 0; q < 8; ++q) v += red[q][i];
+    for (int q = 0; q < warps; ++q) v += red[q][i];
     const int h = i / 3, c = i % 3;
     const int f = 2 * p + h;
     if (f < F) {
@@ -217,7 +237,7 @@ extern "C" int pt_synth_adj_params(int ns, double pixel_scale, int L, int F, con
   if (P2 > 65535) return fail(PT_ERR_UNSUPPORTED, "pt_synth_adj_params: too many frames");
   cudaStream_t s = (cudaStream_t)stream;
   ProfScope ps("k_adj_params", s);
-  k_adj_params<<<dim3(L, P2), 256, 0, s>>>(ns, 1.0 / (ns * pixel_scale), L, F, w,
+  k_adj_params<<<dim3(L, P2), 1024, 0, s>>>(ns, 1.0 / (ns * pixel_scale), L, F, w,
                                            (const float2*)spectra, (const float2*)Z,
                                            (const float2*)ph, out);
   count_launch_a();

@@ -323,12 +323,6 @@ def _synth_frames(grid, sw, shc, sx, sy, crop, n_out, scale):
     return out
 
 
-def _sh_beta(grid):
-    """Grid means of the subharmonic basis rows, (P, 3) complex128 (host)."""
-    x = (np.arange(grid.ns) - grid.ns / 2.0) * grid.dx
-    return np.exp(2j * np.pi * grid._freq[:, :, None] * x[None, None, :]).mean(axis=-1)
-
-
 class _SynthAdjoint:
     """Accumulates the synthesis VJP over chunks of frames (pt_synth_adj_*):
     spectra, weights, shifts and, with subharmonic levels, the level
@@ -348,15 +342,13 @@ class _SynthAdjoint:
         self.shifts = shifts
         self.gSr = (torch.empty((self.L, self.ns, self.ns, 2), dtype=torch.float32,
                                 device=self.dev) if self.need_S else None)
-        self.gw = torch.zeros(self.L, dtype=torch.float64, device=self.dev)
-        self.gsh = torch.zeros((self.F, self.L, 2), dtype=torch.float64, device=self.dev)
+        new = lambda *shape: torch.empty(shape, dtype=torch.float64, device=self.dev)  # noqa: E731
+        self.gw = new(self.L) if self.need_p else None
+        self.gsh = new(self.F, self.L, 2) if self.need_p else None
         self.sh = sh_coef
         if sh_coef is not None:
-            self.fp = torch.as_tensor(grid._freq, dtype=torch.float64, device=self.dev)
-            beta = torch.as_tensor(_sh_beta(grid), device=self.dev)
-            self.bb = beta[:, :, None] * beta[:, None, :]                       # (P, 3, 3)
-            self.cl = sh_coef.detach().to(torch.complex128).permute(1, 0, 2, 3)  # (L, P, 3, 3)
-            self.gc = torch.zeros_like(self.cl)
+            self.shr = torch.view_as_real(sh_coef.detach().contiguous())
+            self.gc = new(self.L, grid.P, 3, 3, 2) if self.need_c else None
         self.first = True
 
     def add(self, f0, g):
@@ -378,39 +370,32 @@ class _SynthAdjoint:
         if self.need_S:
             _lib.call("pt_synth_adj_spectra", ns, L, Fc, _ptr(self.w), _ptr(z), _ptr(ph),
                       int(not self.first), _ptr(self.gSr), s)
+        part = proj = None
         if self.need_p:
             part = torch.empty((L, Fc, 3), dtype=torch.float64, device=self.dev)
             _lib.call("pt_synth_adj_params", ns, grid.dx, L, Fc, _ptr(self.w), _ptr(self.sr),
                       _ptr(z), _ptr(ph), _ptr(part), s)
-            self.gw += part[..., 0].sum(dim=1)
-            self.gsh[f0:f0 + Fc] += part[..., 1:].transpose(0, 1)
         if self.sh is not None and (self.need_p or self.need_c):
-            P = grid.P
-            proj = torch.empty((Fc, 18 * P + 1), dtype=torch.float64, device=self.dev)
+            proj = torch.empty((Fc, 18 * grid.P + 1), dtype=torch.float64, device=self.dev)
             _lib.call("pt_synth_adj_sh", grid.handle, Fc, self.crop, self.n_out, _ptr(g),
                       _ptr(proj), s)
-            G = torch.complex(proj[:, 0:18 * P:2], proj[:, 1:18 * P:2]).reshape(Fc, P, 3, 3)
-            Q = self.scale * (G - self.bb[None] * proj[:, 18 * P, None, None, None])
-            ex = torch.exp(2j * np.pi * sx.double()[:, :, None, None] * self.fp[None, None])
-            ey = torch.exp(2j * np.pi * sy.double()[:, :, None, None] * self.fp[None, None])
-            E = ex[..., :, None] * ey[..., None, :]                             # (Fc, L, P, 3, 3)
-            EQ = E * Q[:, None]
-            if self.need_p:
-                M = self.cl[None] * EQ
-                self.gw += M.real.sum(dim=(0, 2, 3, 4))
-                wMi = (self.w.double()[None, :, None, None, None] * M).imag
-                self.gsh[f0:f0 + Fc, :, 0] -= 2 * np.pi * torch.einsum("pi,flpij->fl", self.fp, wMi)
-                self.gsh[f0:f0 + Fc, :, 1] -= 2 * np.pi * torch.einsum("pj,flpij->fl", self.fp, wMi)
-            if self.need_c:
-                self.gc += torch.conj(self.w.double()[:, None, None, None] * EQ.sum(dim=0))
+        if part is not None or proj is not None:
+            opt = lambda t: None if t is None else _ptr(t)  # noqa: E731
+            nbytes = int(_lib.load().pt_synth_adj_levels_workspace_bytes(
+                L, Fc, grid.P if proj is not None else 0))
+            work = torch.empty(nbytes, dtype=torch.uint8, device=self.dev)
+            _lib.call("pt_synth_adj_levels", grid.handle, L, Fc, int(f0), self.scale, _ptr(self.w),
+                      _ptr(self.shr) if proj is not None else None, _ptr(sx), _ptr(sy), opt(proj),
+                      opt(part), int(not self.first), opt(self.gw), opt(self.gsh),
+                      opt(self.gc) if proj is not None else None, _ptr(work), nbytes, s)
         self.first = False
 
     def grads(self):
         torch = self.torch
         gS = torch.view_as_complex(self.gSr) if self.need_S else None
-        gc = (self.gc.permute(1, 0, 2, 3).to(torch.complex64).contiguous()
+        gc = (torch.view_as_complex(self.gc).permute(1, 0, 2, 3).to(torch.complex64).contiguous()
               if self.sh is not None and self.need_c else None)
-        return gS, self.gw.float(), self.gsh, gc
+        return gS, self.gw.float() if self.need_p else None, self.gsh, gc
 
 
 def _synth_inputs(spectra, weights, sh_coef, shifts, grid, who):
