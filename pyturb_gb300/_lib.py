@@ -190,7 +190,7 @@ def last_error() -> str:
 
 def call(name: str, *args: Any) -> None:
     """Invoke a status-returning entry point; raise on failure."""
-    lib = load()
+    lib = _lib if _lib is not None else load()
     rc = getattr(lib, name)(*args)
     if rc == PT_OK:
         return
@@ -221,4 +221,6 @@ def prof_report() -> dict:
 
 def as_dptr(arr) -> Any:
     """ctypes double* view of a C-contiguous float64 numpy array."""
+    if arr.flags.writeable and arr.size:
+        return (C.c_double * arr.size).from_buffer(arr)  # a third of the cost of data_as
     return arr.ctypes.data_as(dptr)

@@ -19,6 +19,7 @@ rendered one at a time.
 
 from __future__ import annotations
 
+import math
 import warnings
 from typing import Any, Dict, Iterator, List, Optional, Sequence, Tuple
 
@@ -146,6 +147,8 @@ class Atmosphere:
         self._vx = np.asarray(self._vx, dtype=np.float64)
         self._vy = np.asarray(self._vy, dtype=np.float64)
         self._alt = np.asarray(self._alt, dtype=np.float64)
+        self._max_speed = float(np.hypot(self._vx, self._vy).max())
+        self._max_alt = float(np.abs(self._alt).max())
 
         groups: Dict[float, List[int]] = {}
         for i, ly in enumerate(self.layers):
@@ -210,6 +213,7 @@ class Atmosphere:
         streams = [NoiseStream(s, self._host_noise) for s in self._flow_seeds]
         self._spec = SpectralLayers(ns, dx, self._sh_freqs, self._amplitudes_host, sh, streams)
         self._boiling = bool(np.any(np.isfinite(self.tau_boil)))
+        self._min_tau = float(self.tau_boil[np.isfinite(self.tau_boil)].min()) if self._boiling else None
         self._spec_initial = None
         if self._boiling:
             self._spec_initial = (self._spec.spectra.clone(), self._spec.sh_coef.clone())
@@ -295,6 +299,15 @@ class Atmosphere:
             f"({float(disp[tuple(flat)]):.2f} m) exceeds the screen's period "
             f"({self._screen_period_m:.2f} m).", PeriodicWrapWarning, stacklevel=3)
 
+    def _may_wrap(self, t: float, ox: float, oy: float) -> bool:
+        """Whether a layer's displacement can reach the screen period for times up
+        to ``t`` and direction tangents up to ``(ox, oy)`` in size: a cheap bound
+        before :meth:`_check_wrap` looks at each layer."""
+        if self._wrap_warned:
+            return False
+        reach = self._max_speed * t + self._max_alt * math.hypot(ox, oy)
+        return not reach < 0.999999 * self._screen_period_m
+
     def _scale(self, wavelength: Optional[float]) -> float:
         return output_scale(self.wavelength, wavelength, self.dispersion, self.wet_fraction)
 
@@ -304,19 +317,41 @@ class Atmosphere:
         """Frames for (t, ox, oy) triples: (F, n, n), each ``_integrate`` of the reference."""
         disp_x = self._vx[None, :] * times[:, None] + self._alt[None, :] * oxs[:, None]
         disp_y = self._vy[None, :] * times[:, None] + self._alt[None, :] * oys[:, None]
-        if not self._wrap_warned:
+        if times.size and self._may_wrap(float(np.abs(times).max()), float(np.abs(oxs).max()),
+                                         float(np.abs(oys).max())):
             self._check_wrap(disp_x, disp_y)
         if self._lgs_mag is not None:
             torch = torch_module()
             out = torch.empty((len(times), self.n, self.n), dtype=torch.float32,
                               device=self._spec.grid.device)
             for k in range(len(times)):
-                screens = self._spec.layer_screens(disp_x[k], disp_y[k])
-                _lib.call("pt_lgs_zoom", len(self.layers), self.n_screen, self.n,
-                          self._zoom_taps, dptr(self._zoom_idx), dptr(self._zoom_w),
-                          dptr(screens), float(scale), dptr(out[k]), stream_handle())
+                self._zoom(disp_x[k], disp_y[k], scale, out[k])
             return out
         return self._spec.frames(disp_x, disp_y, self.margin_pix, self.n, scale)
+
+    def _frame_at(self, t: float, scale: float):
+        """The on-axis frame ``(n, n)`` at ``t``: one row of :meth:`_phase_frames`
+        without its per-direction tables."""
+        if self.engine != "spectral":
+            self._ext.set_time(t)
+            return self._ext.integrate(scale=scale)
+        disp_x, disp_y = self._vx * t, self._vy * t
+        if self._may_wrap(abs(t), 0.0, 0.0):
+            self._check_wrap(disp_x[None], disp_y[None])
+        if self._lgs_mag is None:
+            return self._spec.frames(disp_x, disp_y, self.margin_pix, self.n, scale)[0]
+        return self._zoom(disp_x, disp_y, scale)
+
+    def _zoom(self, disp_x, disp_y, scale: float, out=None):
+        """The layer screens at one displacement each, through the laser cone."""
+        torch = torch_module()
+        if out is None:
+            out = torch.empty((self.n, self.n), dtype=torch.float32, device=self._spec.grid.device)
+        screens = self._spec.layer_screens(disp_x, disp_y)
+        _lib.call("pt_lgs_zoom", len(self.layers), self.n_screen, self.n, self._zoom_taps,
+                  dptr(self._zoom_idx), dptr(self._zoom_w), dptr(screens), float(scale), dptr(out),
+                  stream_handle())
+        return out
 
     def _phase_frames(self, times, oxs, oys, scale: float):
         if self.engine == "spectral":
@@ -332,10 +367,8 @@ class Atmosphere:
 
     def _boil_step(self, dt: float) -> None:
         """One AR(1) step per Fourier mode (``src/pyturb/atmosphere.py:1092-1126``)."""
-        with np.errstate(divide="ignore"):
-            alpha = np.where(np.isfinite(self.tau_boil), np.exp(-dt / self.tau_boil), 1.0)
-        if np.all(alpha >= 1.0):
-            return
+        if self._min_tau is None or math.exp(-dt / self._min_tau) >= 1.0:
+            return  # no layer boils, or none within float64 of one step
         L, ns, P = len(self.layers), self.n_screen, self.subharmonics
         noise = sh_noise = None
         if self._boil_rng.injected:
@@ -362,7 +395,7 @@ class Atmosphere:
         (``src/pyturb/atmosphere.py:801-869``)."""
         scale = self._scale(wavelength)
         if directions is None:
-            return self._phase_frames([float(t)], [0.0], [0.0], scale)[0]
+            return self._frame_at(float(t), scale)
         oxs, oys = [], []
         for thx, thy in directions:
             radius = float(np.hypot(thx, thy))
@@ -392,7 +425,7 @@ class Atmosphere:
         if not batched:
             for _ in range(steps):
                 t = self._t
-                frame = self._phase_frames([t], [0.0], [0.0], scale)[0]
+                frame = self._frame_at(t, scale)
                 yield t, frame
                 self._t += dt
                 self._after_step(dt)
@@ -472,7 +505,7 @@ class Atmosphere:
         t = np.asarray(times, dtype=np.float64).reshape(-1)
         disp_x = self._vx[None, :] * t[:, None]
         disp_y = self._vy[None, :] * t[:, None]
-        if not self._wrap_warned:
+        if t.size and self._may_wrap(float(np.abs(t).max()), 0.0, 0.0):
             self._check_wrap(disp_x, disp_y)
         return self._spec.frames(disp_x, disp_y, self.margin_pix, self.n,
                                  self._scale(wavelength), out=out)
@@ -500,7 +533,7 @@ class Atmosphere:
             raise ValueError("dt must be positive")
         self._t += float(dt)
         self._after_step(float(dt))
-        return self._phase_frames([self._t], [0.0], [0.0], self._scale(wavelength))[0]
+        return self._frame_at(self._t, self._scale(wavelength))
 
     def _generators(self) -> List[PhaseScreen]:
         if self._sample_generators is None:

@@ -1623,8 +1623,10 @@ extern "C" int pt_ifft2(const pt_grid* g, const float* in, float* out, int batch
   const int ns = g->ns, blen = fft_buf_len(g->desc), ch = gen_chunk(ns),
             rpc = rows_per_cta(blen), C = cols_per_cta(blen);
   const size_t rs = rows_smem(ns, blen, rpc), cs = cols_smem(ns, blen, C, 0);
-  if (int rc = set_smem(k_rows, rs, "k_rows")) return rc;
-  if (int rc = set_smem(k_plain_cols, cs, "k_plain_cols")) return rc;
+  if (!pow2_fast(ns)) {
+    if (int rc = set_smem(k_rows, rs, "k_rows")) return rc;
+    if (int rc = set_smem(k_plain_cols, cs, "k_plain_cols")) return rc;
+  }
   GenRowArgs none{};
   for (int b0 = 0; b0 < batch; b0 += ch) {
     const int nb = std::min(ch, batch - b0);
@@ -1667,8 +1669,10 @@ static int generate_impl(const pt_grid* g, int count, const float* amplitude,
   const int blen = fft_buf_len(g->desc);
   const int ch = gen_chunk(ns), rpc = rows_per_cta(blen), C = cols_per_cta(blen);
   const size_t rs = rows_smem(ns, blen, rpc), cs = cols_smem(ns, blen, C, P);
-  if (int rc = set_smem(k_rows, rs, "k_rows")) return rc;
-  if (int rc = set_smem(k_pair_cols, cs, "k_pair_cols")) return rc;
+  if (!pow2_fast(ns) && !gt_m(ns)) {
+    if (int rc = set_smem(k_rows, rs, "k_rows")) return rc;
+    if (int rc = set_smem(k_pair_cols, cs, "k_pair_cols")) return rc;
+  }
   for (int b0 = 0; b0 < n_fft; b0 += ch) {
     const int nb = std::min(ch, n_fft - b0);
     GenRowArgs ga{amplitude, noise, n_fft, b0, seed, call, sh_amp, sh_noise, g->beta,
@@ -1783,8 +1787,8 @@ extern "C" int pt_frames(const pt_grid* g, int L, const float* spectra, const fl
   const int J = per_layer ? 1 : L;
   if (2 * J > kShiftDoubles) return fail(PT_ERR_UNSUPPORTED, "pt_frames: at most 896 layers");
   const size_t rs = frame_rows_smem(ns, blen), cs = cols_smem(ns, blen, C, P);
-  if (int rc = set_smem(k_frame_rows, rs, "k_frame_rows")) return rc;
-  if (int rc = set_smem(k_pair_cols, cs, "k_pair_cols")) return rc;
+  if (!pow2_fast(ns))
+    if (int rc = set_smem(k_pair_cols, cs, "k_pair_cols")) return rc;
   const int fchunk = 2 * ch;
   const int fsub = std::max(1, kShiftDoubles / (2 * J));  // frames per parameter block
   for (int f0 = 0; f0 < F; f0 += fchunk) {
@@ -1847,6 +1851,7 @@ extern "C" int pt_frames(const pt_grid* g, int L, const float* spectra, const fl
         return rc;
     } else {
       FrameRowArgs fa{(const float2*)spectra, w.px, w.py, J, nf, f0, per_layer};
+      if (int rc = set_smem(k_frame_rows, rs, "k_frame_rows")) return rc;
       ProfScope ps("k_frame_rows", s);
       k_frame_rows<<<dim3(ns / 2 + 1, npair), kThreads, rs, s>>>(fd, g->tw, fa, w.img);
     }

@@ -22,7 +22,7 @@ rotated, magnified, shifted pupil grid and sums the layers
 from __future__ import annotations
 
 import ctypes as C
-from math import floor
+from math import ceil, floor
 from typing import Any, List, Optional, Sequence, Tuple, Union
 
 import numpy as np
@@ -133,6 +133,7 @@ class RingExtruder:
         self.groups = [int(g) for g in groups]
         self.bscale = [float(b) for b in bscale]
         self.streams = list(streams)
+        self._injected = any(st.injected for st in self.streams)
         if device_operator is not None:
             self.M = device_operator if device_operator.dim() == 3 else device_operator[None]
         else:
@@ -164,6 +165,7 @@ class RingExtruder:
         self._key = np.asarray([st.key for st in self.streams], dtype=np.uint64)
         self.work_bytes = 0
         self.work = None
+        self._work_for: set = set()
         self.tiles = None
         if self.terms:
             # the operator split into bf16 terms, tiled for the tensor cores (once)
@@ -174,6 +176,8 @@ class RingExtruder:
                       self.terms, dptr(self.tiles), nbytes, stream_handle())
 
     def _ensure_work(self, jobs_per_step: int) -> None:
+        if jobs_per_step in self._work_for:
+            return
         lib = _lib.load()
         if self.terms:
             need = int(lib.pt_extrude_tc_workspace_bytes(self.W, self.m, self.ns,
@@ -185,6 +189,7 @@ class RingExtruder:
             torch = torch_module()
             self.work = torch.empty(need, dtype=torch.uint8, device=cuda_device())
             self.work_bytes = need
+        self._work_for.add(jobs_per_step)  # the workspace only grows
 
     def seed_rows(self, s: int, rows) -> None:
         """Copy the initial (span, W) rows of screen s into ring rows [0, span)."""
@@ -200,11 +205,11 @@ class RingExtruder:
         if steps <= 0:
             return
         noise = None
-        if any(st.injected for st in self.streams):
+        if self._injected:
             rows = [self.streams[s].draw((self.W,))
                     for k in range(steps) for s in range(self.S) if k < counts[s]]
             noise = upload(np.stack(rows))
-        self._ensure_work(int((counts > 0).sum()))
+        self._ensure_work(int(np.count_nonzero(counts > 0)))
         ptr = lambda a: a.ctypes.data  # noqa: E731
         if self.terms:
             _lib.call("pt_extrude_batch_tc", self.W, self.m, self._sp, int(self.increments),
@@ -337,6 +342,7 @@ class ExtrudedAtmosphere:
             groups.append(op_index[key])
         streams = [NoiseStream(s, host_noise) for s in config.seeds]
         self._streams = streams
+        self._readout_fixed = None
         self.layers: List[_LayerGeom] = []
         for (vx, vy), alt, mag, fov in zip(config.layer_wind, config.layer_altitude_los, mags,
                                            config.field_of_view_pix):
@@ -392,7 +398,7 @@ class ExtrudedAtmosphere:
     def _plan(self, ly: _LayerGeom) -> int:
         """Rows the layer needs to cover its travel, with the reference's
         compaction bookkeeping applied (``src/pyturb/extrude.py:424-449``)."""
-        top = int(np.ceil(ly.along_max + ly.fov + ly.travel)) + 2
+        top = ceil(ly.along_max + ly.fov + ly.travel) + 2
         count = 0
         while ly.base + ly.fill - 1 < top:
             if ly.fill == self.capacity:
@@ -477,16 +483,19 @@ class ExtrudedAtmosphere:
                       a, b, dptr(scr.buf[q]), stream_handle())
 
     def readout_params(self, thx: float = 0.0, thy: float = 0.0):
-        arr = (_lib.ReadoutLayer * len(self.layers))()
-        for i, ly in enumerate(self.layers):
-            off_a, off_p = ly.offsets_for_direction(thx, thy)
-            p = arr[i]
-            p.screen = i
+        if self._readout_fixed is None:  # what does not move: filled once, copied a call
+            fixed = (_lib.ReadoutLayer * len(self.layers))()
+            for i, ly in enumerate(self.layers):
+                p = fixed[i]
+                p.screen, p.cos_t, p.sin_t, p.mag = i, ly.cos, ly.sin, ly.mag
+            self._readout_fixed = fixed
+        arr = type(self._readout_fixed).from_buffer_copy(self._readout_fixed)
+        cap = self.capacity
+        axis = thx == 0.0 and thy == 0.0
+        for p, ly in zip(arr, self.layers):
+            off_a, off_p = (0.0, 0.0) if axis else ly.offsets_for_direction(thx, thy)
             p.row_max = ly.fill - 1
-            p.anchor_phys = (ly.base - ly.v0) % self.capacity
-            p.cos_t = ly.cos
-            p.sin_t = ly.sin
-            p.mag = ly.mag
+            p.anchor_phys = (ly.base - ly.v0) % cap
             p.shift_along = (ly.travel - ly.base) + off_a
             p.shift_perp = off_p
         return arr
