@@ -332,22 +332,25 @@ __device__ __forceinline__ void two_sum_acc(float& s, float& c, float h) {
 
 // The anchor's projections as one small double-float GEMM over the
 // concatenated columns [stencil (Kz) | noise (W) | new row (W)]:
-//   part[z][j][i] = sum over slice z of P'[i][k] x'_j[k],
+//   part[j][z][i] = sum over slice z of P'[i][k] x'_j[k],
 //   P' = [U^T A | U^T B | -U],  x'_j = [X_j[0, Kz) | X_j[Kz, K) | new_j],
 // so d = sum_z part is U^T A z + U^T B (bscale beta) - U^T new. The table
 // P'^T is prepared once on the host as (hi, lo) float32 rows of R values per
-// column k, the modes of a row stored in pairs (i, i + 16), so a chunk of 64
-// columns is one contiguous copy. A CTA takes 16 jobs x all R modes over one
-// K slice (each thread one job and R/16 modes), staging 64-column chunks of
-// x' and P' in shared memory; part holds (s, c) double-float pairs.
-template <int R>
+// column k, the modes of a row stored in pairs (i, i + 16), so a chunk of 32
+// columns is one contiguous copy. A CTA takes JT jobs x all R modes over one
+// K slice (each thread a mode pair and JT R / 512 jobs), staging 32-column
+// chunks of x' and P' in shared memory; part holds (s, c) double-float pairs.
+// The bound is the FP32 pipe (eleven packed operations a double-float product),
+// so JT is the width of 64, 48 or 32 that pads the jobs least: 144 jobs, R = 64,
+// W = 1449: 32.8 us at 64, 27.9 us at 48.
+template <int R, int JT>
 __global__ void __launch_bounds__(256)
 k_anchor_gemm(int W, int K, int Kz, int cap, int g, int J, int kslice, int incr,
               const RingDst dst, const float* __restrict__ X, const AnchorDev an,
               const float* __restrict__ buf, float2* __restrict__ part) {
   // 32-column chunks keep the static shared memory under 48 KB; the operand
   // is staged as (x, x) pairs, ready for the packed products
-  constexpr int KC = 32, NP2 = R / 2, JT = 64, JPT = JT * NP2 / 256;
+  constexpr int KC = 32, NP2 = R / 2, JPT = JT * NP2 / 256;
   __shared__ f2p xs[JT][KC + 1];
   __shared__ f2p phs[KC][NP2], pls[KC][NP2];
   const int tid = threadIdx.x;
@@ -406,51 +409,98 @@ k_anchor_gemm(int W, int K, int Kz, int cap, int g, int J, int kslice, int incr,
     float s0, s1, c0, c1;
     unpack2(s[q], s0, s1);
     unpack2(c[q], c0, c1);
-    part[((size_t)z * J + j) * R + i0] = make_float2(s0, c0);
-    part[((size_t)z * J + j) * R + i0 + 16] = make_float2(s1, c1);
+    float2* dst_j = part + ((size_t)j * gridDim.y + z) * R;  // a job's slices lie together
+    dst_j[i0] = make_float2(s0, c0);
+    dst_j[i0 + 16] = make_float2(s1, c1);
   }
 }
 
-// new row += U d, d = sum over the slices of part (fixed order), one CTA per
-// job: warp w reduces modes w, w + 8, ... (lanes over slices, then a fixed
-// butterfly), then every thread corrects its pixels.
+// d[0, R) of one job, the sum of its Z shares in a fixed order, by 1024 threads: a
+// warp takes every 32nd share of the R modes, coalesced and all in flight; a
+// warp a mode adds the 32 sums by a fixed butterfly. Ends with a barrier.
 template <int R>
-__global__ void __launch_bounds__(256)
-k_anchor_apply(int W, int cap, int J, int nsplit, const RingDst dst,
-               const float2* __restrict__ part, const float* __restrict__ u,
-               float* __restrict__ buf) {
-  __shared__ float ds[R];
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int j = blockIdx.x;
-  if (j >= J) return;
-  for (int i = warp; i < R; i += 8) {
-    float ss = 0.f, cc = 0.f;
-    for (int z = lane; z < nsplit; z += 32) {
-      const float2 q = part[((size_t)z * J + j) * R + i];
-      cc = __fadd_rn(cc, q.y);
-      two_sum_acc(ss, cc, q.x);
-    }
+__device__ __forceinline__ void anchor_sum(const float2* __restrict__ pj, int Z, float* ds) {
+  __shared__ float2 sum[32][R + 1];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      const float so = __shfl_xor_sync(0xffffffffu, ss, o);
-      const float co = __shfl_xor_sync(0xffffffffu, cc, o);
-      // the same operands in the same order on both lanes of a pair
-      const float a = (lane & o) ? so : ss, b = (lane & o) ? ss : so;
-      float s2 = a, c2 = (lane & o) ? __fadd_rn(co, cc) : __fadd_rn(cc, co);
-      two_sum_acc(s2, c2, b);
-      ss = s2;
-      cc = c2;
+  for (int b = 0; b < R; b += 32) {
+    float s = 0.f, c = 0.f;
+#pragma unroll 10
+    for (int z = warp; z < Z; z += 32) {
+      const float2 v = pj[(size_t)z * R + b + lane];
+      c = __fadd_rn(c, v.y);
+      two_sum_acc(s, c, v.x);
     }
-    if (lane == 0) ds[i] = ss + cc;
+    sum[warp][b + lane] = make_float2(s, c);
   }
   __syncthreads();
-  float* row = buf + ((size_t)dst.d[j].x * cap + dst.d[j].y) * W;
-  for (int w = tid; w < W; w += 256) {
-    float v = 0.f;
 #pragma unroll
-    for (int i = 0; i < R; ++i) v = fmaf(__ldg(u + (size_t)i * W + w), ds[i], v);
-    row[w] += v;
+  for (int i = warp; i < R; i += 32) {
+    float s = sum[lane][i].x, c = sum[lane][i].y;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      const float so = __shfl_xor_sync(0xffffffffu, s, o);
+      const float co = __shfl_xor_sync(0xffffffffu, c, o);
+      // the same operands in the same order on both lanes of a pair
+      float s2 = (lane & o) ? so : s, c2 = (lane & o) ? __fadd_rn(co, c) : __fadd_rn(c, co);
+      two_sum_acc(s2, c2, (lane & o) ? s : so);
+      s = s2;
+      c = c2;
+    }
+    if (lane == 0) ds[i] = s + c;
   }
+  __syncthreads();
+}
+
+// Few jobs: new row += U d in one launch, a CTA a job and 1024 pixels.
+template <int R>
+__global__ void __launch_bounds__(1024)
+k_anchor_apply(int W, int cap, int Z, const RingDst dst, const float2* __restrict__ part,
+               const float* __restrict__ u, float* __restrict__ buf) {
+  __shared__ float ds[R];
+  const int j = blockIdx.y, w = blockIdx.x * 1024 + threadIdx.x;
+  anchor_sum<R>(part + (size_t)j * Z * R, Z, ds);
+  if (w >= W) return;
+  float v = 0.f;
+#pragma unroll
+  for (int i = 0; i < R; ++i) v = fmaf(__ldg(u + (size_t)i * W + w), ds[i], v);
+  buf[((size_t)dst.d[j].x * cap + dst.d[j].y) * W + w] += v;
+}
+
+// Many jobs: the sums to d (J, R), then kAddJobs jobs a CTA share each value of
+// U, which a CTA a job would read J times over from L2. 144 jobs, 64 modes, 182
+// shares, W = 1449: 25.8 us with a job's shares scattered over the slices and a
+// lane a share, 15.3 us by k_anchor_apply, 13.5 us so.
+template <int R>
+__global__ void __launch_bounds__(1024)
+k_anchor_sum(int Z, const float2* __restrict__ part, float* __restrict__ d) {
+  __shared__ float ds[R];
+  anchor_sum<R>(part + (size_t)blockIdx.x * Z * R, Z, ds);
+  if (threadIdx.x < R) d[(size_t)blockIdx.x * R + threadIdx.x] = ds[threadIdx.x];
+}
+constexpr int kAddJobs = 8;
+template <int R>
+__global__ void __launch_bounds__(128)
+k_anchor_add(int W, int cap, int J, const RingDst dst, const float* __restrict__ d,
+             const float* __restrict__ u, float* __restrict__ buf) {
+  __shared__ __align__(16) float ds[R][kAddJobs];
+  const int j0 = blockIdx.y * kAddJobs, w = blockIdx.x * 128 + threadIdx.x;
+  for (int e = threadIdx.x; e < R * kAddJobs; e += 128)
+    ds[e % R][e / R] = j0 + e / R < J ? d[(size_t)(j0 + e / R) * R + e % R] : 0.f;
+  __syncthreads();
+  if (w >= W) return;
+  float v[kAddJobs];
+#pragma unroll
+  for (int q = 0; q < kAddJobs; ++q) v[q] = 0.f;
+#pragma unroll 32
+  for (int i = 0; i < R; ++i) {
+    const float ui = __ldg(u + (size_t)i * W + w);
+#pragma unroll
+    for (int q = 0; q < kAddJobs; ++q) v[q] = fmaf(ui, ds[i][q], v[q]);
+  }
+#pragma unroll
+  for (int q = 0; q < kAddJobs; ++q)
+    if (j0 + q < J) buf[((size_t)dst.d[j0 + q].x * cap + dst.d[j0 + q].y) * W + w] += v[q];
 }
 
 // partial[z][j][r] = sum_{k in slice z} M[r][k] X[j][k]
@@ -614,7 +664,7 @@ __global__ void k_extrude_reduce(int W, int J, int cap, int nsplit, const float*
 // the rings, its warps split K, and the sums end in the ring without slices in
 // memory; the CTA also adds its share of the anchor's projections (a slice of
 // the operand columns, and its own new pixels) and makes its share of the next
-// launch's noise. k_step_anchor sums the shares and corrects the rows. So the
+// launch's noise. k_anchor_apply sums the shares and corrects the rows. So the
 // same step takes 11 us + 5 us (both latency: the operand's way through L2, the
 // reduction, the anchor's double-float chains). More than kStepJobs screens, or
 // an operand beyond shared memory, leave the product to the tiled GEMM, which
@@ -800,53 +850,6 @@ k_row_step(const StepArgs a, const StepJobs jobs, const StepJobs next) {
     dst[i0] = make_float2(s0, e0);
     dst[i0 + 16] = make_float2(s1, e1);
   }
-}
-
-// new row += U d, d the sum of the Z shares of a job in a fixed order: a warp
-// takes every 32nd share of the R modes, coalesced and all in flight; then a
-// warp a mode adds the 32 sums by a fixed butterfly.
-template <int R>
-__global__ void __launch_bounds__(1024)
-k_step_anchor(int W, int cap, int Z, const StepJobs jobs, const float2* __restrict__ part,
-              const float* __restrict__ u, float* __restrict__ buf) {
-  __shared__ float2 sum[32][R + 1];
-  __shared__ float ds[R];
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int j = blockIdx.y, w = blockIdx.x * 1024 + tid;
-  const float2* pj = part + (size_t)j * Z * R;
-#pragma unroll
-  for (int b = 0; b < R; b += 32) {
-    float s = 0.f, c = 0.f;
-#pragma unroll 10
-    for (int z = warp; z < Z; z += 32) {
-      const float2 q = pj[(size_t)z * R + b + lane];
-      c = __fadd_rn(c, q.y);
-      two_sum_acc(s, c, q.x);
-    }
-    sum[warp][b + lane] = make_float2(s, c);
-  }
-  __syncthreads();
-#pragma unroll
-  for (int i = warp; i < R; i += 32) {
-    float s = sum[lane][i].x, c = sum[lane][i].y;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      const float so = __shfl_xor_sync(0xffffffffu, s, o);
-      const float co = __shfl_xor_sync(0xffffffffu, c, o);
-      // the same operands in the same order on both lanes of a pair
-      float s2 = (lane & o) ? so : s, c2 = (lane & o) ? __fadd_rn(co, c) : __fadd_rn(c, co);
-      two_sum_acc(s2, c2, (lane & o) ? s : so);
-      s = s2;
-      c = c2;
-    }
-    if (lane == 0) ds[i] = s + c;
-  }
-  __syncthreads();
-  if (w >= W) return;
-  float v = 0.f;
-#pragma unroll
-  for (int i = 0; i < R; ++i) v = fmaf(__ldg(u + (size_t)i * W + w), ds[i], v);
-  buf[((size_t)jobs.screen[j] * cap + jobs.head[j]) * W + w] += v;
 }
 
 // CTAs of a row step: one per SM, or fewer
@@ -1137,7 +1140,7 @@ struct ExtrudeForm {
   int incr;                // the operator is in increment form
 };
 
-// Row steps of few screens: one k_row_step (and k_step_anchor) for the jobs of
+// Row steps of few screens: one k_row_step (and k_anchor_apply) for the jobs of
 // each (step, group), in the workspace [noise (2, J, W) in the operand's place |
 // ... | shares in the partials' place].
 static int step_jobs(const char* who, const ExtrudeForm& form, int W, int m, int cap, float* buf,
@@ -1206,12 +1209,14 @@ static int step_jobs(const char* who, const ExtrudeForm& form, int W, int m, int
     }
     count_launch_e();
     if (R) {
-      ProfScope ps("k_step_anchor", s);
+      ProfScope ps("k_anchor_apply", s);
       const dim3 grid((W + 1023) / 1024, cur.n);
+      RingDst dst{};
+      for (int q = 0; q < cur.n; ++q) dst.d[q] = make_int2(cur.screen[q], cur.head[q]);
       if (R == 32)
-        k_step_anchor<32><<<grid, 1024, 0, s>>>(W, cap, 2 * ctas, cur, a.part, form.anchor->u, buf);
+        k_anchor_apply<32><<<grid, 1024, 0, s>>>(W, cap, 2 * ctas, dst, a.part, form.anchor->u, buf);
       else
-        k_step_anchor<64><<<grid, 1024, 0, s>>>(W, cap, 2 * ctas, cur, a.part, form.anchor->u, buf);
+        k_anchor_apply<64><<<grid, 1024, 0, s>>>(W, cap, 2 * ctas, dst, a.part, form.anchor->u, buf);
       count_launch_e();
     }
     if (int rc = check_launch(who)) return rc;
@@ -1371,7 +1376,11 @@ static int extrude_jobs(const char* who, const ExtrudeForm& form, int W, int m,
           const AnchorDev an{(const f2p*)form.anchor->t_hi, (const f2p*)form.anchor->t_lo,
                              form.anchor->u};
           const int R = form.anchor->modes, Kt = K + (form.incr ? 2 : 1) * W;
-          const int jb = (J + 63) / 64;
+          // the job tile that pads least (the widest of equals)
+          int jt = 64;
+          for (int t : {48, 32})
+            if ((J + t - 1) / t * t < (J + jt - 1) / jt * jt) jt = t;
+          const int jb = (J + jt - 1) / jt;
           // about four CTAs per SM (a single wave of two left SMs idle in its
           // tail), slices of 32 or more columns
           const int nsplit = std::max(1, std::min(std::min(kAnchorSplit, (Kt + 31) / 32),
@@ -1382,18 +1391,33 @@ static int extrude_jobs(const char* who, const ExtrudeForm& form, int W, int m,
               (float2*)((char*)partial + al256((size_t)fw.max_nz * J * W * sizeof(float)));
           {
             ProfScope ps("k_anchor", s);
+            auto go = [&](auto kern) {
+              kern<<<dim3(jb, nz_a), 256, 0, s>>>(W, K, Kz, cap, kv.first, J, kslice, form.incr, dst,
+                                                  X, an, buf, apart);
+            };
             if (R == 32) {
-              k_anchor_gemm<32><<<dim3(jb, nz_a), 256, 0, s>>>(W, K, Kz, cap, kv.first, J,
-                                                               kslice, form.incr, dst, X, an, buf,
-                                                               apart);
-              k_anchor_apply<32><<<J, 256, 0, s>>>(W, cap, J, nz_a, dst, apart, an.u, buf);
+              if (jt == 64) go(k_anchor_gemm<32, 64>);
+              else if (jt == 48) go(k_anchor_gemm<32, 48>);
+              else go(k_anchor_gemm<32, 32>);
             } else {
-              k_anchor_gemm<64><<<dim3(jb, nz_a), 256, 0, s>>>(W, K, Kz, cap, kv.first, J,
-                                                               kslice, form.incr, dst, X, an, buf,
-                                                               apart);
-              k_anchor_apply<64><<<J, 256, 0, s>>>(W, cap, J, nz_a, dst, apart, an.u, buf);
+              if (jt == 64) go(k_anchor_gemm<64, 64>);
+              else if (jt == 48) go(k_anchor_gemm<64, 48>);
+              else go(k_anchor_gemm<64, 32>);
             }
           }
+          {
+            // the operand is spent: its place holds the sums (R <= W modes a job)
+            ProfScope ps("k_anchor_add", s);
+            const dim3 grid((W + 127) / 128, (J + kAddJobs - 1) / kAddJobs);
+            if (R == 32) {
+              k_anchor_sum<32><<<J, 1024, 0, s>>>(nz_a, apart, X);
+              k_anchor_add<32><<<grid, 128, 0, s>>>(W, cap, J, dst, X, an.u, buf);
+            } else {
+              k_anchor_sum<64><<<J, 1024, 0, s>>>(nz_a, apart, X);
+              k_anchor_add<64><<<grid, 128, 0, s>>>(W, cap, J, dst, X, an.u, buf);
+            }
+          }
+          count_launch_e();
           count_launch_e(2);
         }
         count_launch_e(form.terms ? 1 : 2);
