@@ -138,6 +138,9 @@ k_tc_gemm(int W, int J, int NP, int nkc, int cps, int stages, const uint8_t* __r
   const int MT = gridDim.x;
   const int kc0 = z * cps, kc1 = min(nkc, kc0 + cps);
   const int n = kc1 - kc0;
+  // the float32 form's product runs beside this one (it waits for this grid's end
+  // itself); a no-op without a dependent
+  asm volatile("griddepcontrol.launch_dependents;");
   const uint32_t bytesA = TERMS * kTcTileA, bytesB = TERMS * NP * kTcKc * 2;
   const uint32_t stage_bytes = bytesA + bytesB;
   if (warp == 0) tc::tmem_alloc(&tslot, 256);
@@ -239,6 +242,8 @@ TcShape tc_shape(int W, int K, int J, int terms) {
   // one CTA per SM with as many stages as fit in 227 KB (less static shared
   // memory and the 1 KB alignment pad)
   t.stages = (int)std::min<size_t>(kTcMaxStages, (kTcSmemMax - 2048) / t.stage_bytes);
+  // the one-term form shares its SM with a CTA of the FP32 product (36 KB)
+  if (terms == 1) t.stages = (int)std::min<size_t>(t.stages, std::max<size_t>(2, 180 * 1024 / t.stage_bytes));
   return t;
 }
 int tc_max_jobs(int terms) { return terms == 3 ? 160 : 192; }
