@@ -560,9 +560,10 @@ k_extrude_gemm(int W, int K, int J, int kslice, const float* __restrict__ M,
 // and TJ broadcast loads of X feed 8 TJ FMAs. Both operands are row-major with
 // an odd K (no 16-byte alignment), so each stage is read with coalesced
 // scalar loads into registers while the previous stage is multiplied, then
-// stored K-major into the other shared buffer.
+// stored K-major into the other shared buffer. (Packed f32x2 products measured
+// 58 us against 51 us at W = 1449, 144 jobs: they take two pipe cycles each.)
 template <int TJ>
-__global__ void __launch_bounds__(256, TJ >= 9 ? 1 : 2)
+__global__ void __launch_bounds__(256, 2)
 k_extrude_gemm_tiled(int W, int K, int J, int kslice, const float* __restrict__ M,
                      const float* __restrict__ X, float* __restrict__ partial) {
   constexpr int BJ = 16 * TJ;
@@ -636,6 +637,101 @@ k_extrude_gemm_tiled(int W, int K, int J, int kslice, const float* __restrict__ 
     for (int v = 0; v < TJ; ++v) {
       const int j = j0 + tj * TJ + v;
       if (r < W && j < J) pz[(size_t)j * W + r] = acc[u][v];
+    }
+  }
+  // launched beside the correction product: done only when that is
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
+// The product for more than 64 jobs: 512 threads, a warp 128 rows (four a lane)
+// x TJ jobs, so an SM has sixteen warps to cover the shared loads with where the
+// 8 x TJ tiles above leave it eight; a K value costs one 128-bit load of A and
+// TP / 4 broadcast loads of X for 4 TJ products. Slices are written 32
+// consecutive values at a time, through a warp's own shared row. Sums run in the
+// same order. W = 1449, 144 jobs, started beside the correction: 58.4 us with 8 x 9
+// tiles, 54.5 us so.
+template <int TJ>
+__global__ void __launch_bounds__(512, 1)
+k_extrude_gemm_wide(int W, int K, int J, int kslice, const float* __restrict__ M,
+                    const float* __restrict__ X, float* __restrict__ partial) {
+  constexpr int BJ = 16 * TJ, TP = (TJ + 3) & ~3;
+  constexpr int AP = kGBM + 4, XP = 16 * TP + 4, NX = (BJ + 31) / 32;
+  __shared__ __align__(16) float sA[2][kGBK][AP];
+  __shared__ __align__(16) float sX[2][kGBK][XP];
+  const int tid = threadIdx.x, lane = tid & 31, tj = tid >> 5;
+  const int r0 = blockIdx.x * kGBM, j0 = blockIdx.y * BJ;
+  const int kb = blockIdx.z * kslice, ke = min(K, kb + kslice);
+  // staging map: K offset lk, rows / jobs lr + 32 i
+  const int lk = tid & 15, lr = tid >> 4;
+  const uint64_t pol = l2_evict_last();  // the operator is re-read every row step
+  float ra[4], rx[NX];
+  auto load = [&](int k0) {
+    const int k = k0 + lk;
+    const bool kin = k < ke;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int r = r0 + lr + 32 * i;
+      ra[i] = (kin && r < W) ? ld_keep(M + (size_t)r * K + k, pol) : 0.f;
+    }
+#pragma unroll
+    for (int v = 0; v < NX; ++v) {
+      const int j = j0 + lr + 32 * v;
+      rx[v] = (kin && lr + 32 * v < BJ && j < J) ? __ldg(X + (size_t)j * K + k) : 0.f;
+    }
+  };
+  auto store = [&](int b) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) sA[b][lk][lr + 32 * i] = ra[i];
+#pragma unroll
+    for (int v = 0; v < NX; ++v) {
+      const int e = lr + 32 * v;
+      if (e < BJ) sX[b][lk][e / TJ * TP + e % TJ] = rx[v];
+    }
+  };
+  float acc[4][TJ];
+#pragma unroll
+  for (int u = 0; u < 4; ++u)
+#pragma unroll
+    for (int v = 0; v < TJ; ++v) acc[u][v] = 0.f;
+  load(kb);
+  store(0);
+  __syncthreads();
+  int b = 0;
+  for (int k0 = kb; k0 < ke; k0 += kGBK) {
+    const bool more = k0 + kGBK < ke;
+    if (more) load(k0 + kGBK);
+#pragma unroll
+    for (int kk = 0; kk < kGBK; ++kk) {
+      const float4 a4 = *(const float4*)&sA[b][kk][lane * 4];
+      const float a[4] = {a4.x, a4.y, a4.z, a4.w};
+      float x[TP];
+#pragma unroll
+      for (int v = 0; v < TP; v += 4) *(float4*)(x + v) = *(const float4*)&sX[b][kk][tj * TP + v];
+#pragma unroll
+      for (int u = 0; u < 4; ++u)
+#pragma unroll
+        for (int v = 0; v < TJ; ++v) acc[u][v] = fmaf(a[u], x[v], acc[u][v]);
+    }
+    // the other buffer was last read before the previous barrier
+    if (more) store(b ^ 1);
+    __syncthreads();
+    b ^= 1;
+  }
+  float* row = &sA[0][0][0] + tj * kGBM;  // this warp's 128 values (the buffers are spent)
+  static_assert(16 * kGBM <= 2 * kGBK * AP, "output rows fit the A buffers");
+  float* pz = partial + (size_t)blockIdx.z * J * W;
+#pragma unroll
+  for (int v = 0; v < TJ; ++v) {
+    const int j = j0 + tj * TJ + v;
+    __syncwarp();
+    *(float4*)(row + lane * 4) = make_float4(acc[0][v], acc[1][v], acc[2][v], acc[3][v]);
+    __syncwarp();
+    if (j < J) {
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const int r = r0 + 32 * u + lane;
+        if (r < W) pz[(size_t)j * W + r] = row[32 * u + lane];
+      }
     }
   }
   // launched beside the correction product: done only when that is
@@ -1079,10 +1175,10 @@ static int tiled_split(int W, int J, int K) {
   return std::max(1, std::min(s, K / (8 * kGBK)));
 }
 // With `beside` the GEMM is a programmatic dependent of the correction product
-// before it on the stream, which it does not read: the two run side by side (the
-// FP32 product's CTAs leave an SM the registers and shared memory of one more),
-// and the GEMM's CTAs wait for the correction before they end, so that what
-// follows finds both done. 9.5 us a row step beside 51 us at W = 1449, 144 jobs.
+// before it on the stream, which it does not read: the two run side by side as far
+// as the SMs have room, and the GEMM's CTAs wait for the correction before they
+// end, so that what follows finds both done. A row step with the sparse stencil at
+// W = 1449, 144 jobs: 3.7 us shorter.
 static int launch_gemm_tiled(int W, int K, int J, const float* M, const float* X, float* partial,
                              bool beside, int* nz_out, cudaStream_t s) {
   const int tj = tiled_tj(J), bj = 16 * tj;
@@ -1091,10 +1187,10 @@ static int launch_gemm_tiled(int W, int K, int J, const float* M, const float* X
   const int nz = (K + kslice - 1) / kslice;
   const dim3 grid((W + kGBM - 1) / kGBM, (J + bj - 1) / bj, nz);
   ProfScope ps("k_extrude_gemm", s);
-  auto go = [&](auto kern) -> int {
+  auto go = [&](auto kern, int threads) -> int {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
-    cfg.blockDim = dim3(256);
+    cfg.blockDim = dim3(threads);
     cfg.stream = s;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -1103,8 +1199,8 @@ static int launch_gemm_tiled(int W, int K, int J, const float* M, const float* X
     cfg.numAttrs = beside ? 1 : 0;
     return check_cuda(cudaLaunchKernelEx(&cfg, kern, W, K, J, kslice, M, X, partial), "k_extrude_gemm");
   };
-  if (int rc = tj == 2 ? go(k_extrude_gemm_tiled<2>)
-                       : tj == 4 ? go(k_extrude_gemm_tiled<4>) : go(k_extrude_gemm_tiled<9>))
+  if (int rc = tj == 2 ? go(k_extrude_gemm_tiled<2>, 256)
+                       : tj == 4 ? go(k_extrude_gemm_tiled<4>, 256) : go(k_extrude_gemm_wide<9>, 512))
     return rc;
   *nz_out = nz;
   return PT_OK;

@@ -242,7 +242,7 @@ TcShape tc_shape(int W, int K, int J, int terms) {
   // one CTA per SM with as many stages as fit in 227 KB (less static shared
   // memory and the 1 KB alignment pad)
   t.stages = (int)std::min<size_t>(kTcMaxStages, (kTcSmemMax - 2048) / t.stage_bytes);
-  // the one-term form shares its SM with a CTA of the FP32 product (36 KB)
+  // the one-term form leaves its SM room for a CTA of the FP32 product (42 KB)
   if (terms == 1) t.stages = (int)std::min<size_t>(t.stages, std::max<size_t>(2, 180 * 1024 / t.stage_bytes));
   return t;
 }
