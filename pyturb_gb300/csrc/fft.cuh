@@ -1,4 +1,4 @@
-// Shared-memory Stockham autosort FFT (mixed radix 8/4/2/3/5/7 plus a
+// Shared-memory Stockham autosort FFT (mixed radix 8/4/2/3/5/7/11/13 plus a
 // direct-sum stage for any larger prime factor), inverse sign, unnormalised:
 //   X[k] = sum_j x[j] exp(+2 pi i j k / n)
 // which is numpy.fft.ifft(x) * n. Every transform of a pass lives in shared
@@ -130,20 +130,77 @@ __device__ __forceinline__ void bfly5(float2* v) {
   v[3] = csub(m2, r2);
 }
 
-// Generic small radix (7): direct sum with the transform's own twiddle table.
+// Prime radices 7, 11 and 13 from the sums and differences of the conjugate input
+// pairs: with t_j = v_j + v_{R-j}, d_j = v_j - v_{R-j},
+//   out_{q, R-q} = v_0 + sum_j cos(2 pi j q / R) t_j +- i sum_j sin(2 pi j q / R) d_j,
+// (R - 1) / 2 real coefficients an output component instead of R - 1 complex
+// products. As a direct sum over shared memory a radix-13 stage was most of a
+// 728-point transform: paired columns of three 728^2 images 62.7 us so, 41.4 us
+// with this butterfly.
 template <int R>
-__device__ __forceinline__ void bfly_direct(float2* v, const float2* tw, int n) {
-  float2 o[R];
-  const int step = n / R;
+struct OddRoots;  // cos and sin of 2 pi k / R, k = 1 .. (R - 1) / 2
+template <>
+struct OddRoots<7> {
+  static __device__ __forceinline__ float c(int k) {
+    constexpr float t[] = {0.62348980185873359f, -0.22252093395631434f, -0.90096886790241903f};
+    return t[k];
+  }
+  static __device__ __forceinline__ float s(int k) {
+    constexpr float t[] = {0.7818314824680298f, 0.97492791218182362f, 0.43388373911755823f};
+    return t[k];
+  }
+};
+template <>
+struct OddRoots<11> {
+  static __device__ __forceinline__ float c(int k) {
+    constexpr float t[] = {0.84125353283118121f, 0.41541501300188644f, -0.142314838273285f, -0.65486073394528499f, -0.95949297361449737f};
+    return t[k];
+  }
+  static __device__ __forceinline__ float s(int k) {
+    constexpr float t[] = {0.54064081745559756f, 0.90963199535451833f, 0.9898214418809328f, 0.75574957435425827f, 0.28173255684142967f};
+    return t[k];
+  }
+};
+template <>
+struct OddRoots<13> {
+  static __device__ __forceinline__ float c(int k) {
+    constexpr float t[] = {0.88545602565320991f, 0.56806474673115592f, 0.12053668025532301f, -0.35460488704253545f, -0.74851074817110119f, -0.97094181742605201f};
+    return t[k];
+  }
+  static __device__ __forceinline__ float s(int k) {
+    constexpr float t[] = {0.46472317204376851f, 0.82298386589365635f, 0.99270887409805397f, 0.93501624268541483f, 0.66312265824079519f, 0.23931566428755768f};
+    return t[k];
+  }
+};
+template <int R>
+__device__ __forceinline__ void bfly_odd(float2* v) {
+  constexpr int H = (R - 1) / 2;
+  float2 t[H], d[H];
+  float2 sum = v[0];
 #pragma unroll
-  for (int q = 0; q < R; ++q) {
-    float2 acc = v[0];
-#pragma unroll
-    for (int r = 1; r < R; ++r) acc = cfma(v[r], tw[((q * r) % R) * step], acc);
-    o[q] = acc;
+  for (int j = 1; j <= H; ++j) {
+    t[j - 1] = cadd(v[j], v[R - j]);
+    d[j - 1] = csub(v[j], v[R - j]);
+    sum = cadd(sum, t[j - 1]);
   }
 #pragma unroll
-  for (int q = 0; q < R; ++q) v[q] = o[q];
+  for (int q = 1; q <= H; ++q) {
+    float2 m = v[0], r = make_float2(0.f, 0.f);
+#pragma unroll
+    for (int j = 1; j <= H; ++j) {
+      const int e = j * q % R;  // cos is even, sin odd about R / 2
+      const float c = OddRoots<R>::c((e <= H ? e : R - e) - 1);
+      const float sn = e <= H ? OddRoots<R>::s(e - 1) : -OddRoots<R>::s(R - e - 1);
+      m.x = fmaf(c, t[j - 1].x, m.x);
+      m.y = fmaf(c, t[j - 1].y, m.y);
+      r.x = fmaf(-sn, d[j - 1].y, r.x);
+      r.y = fmaf(sn, d[j - 1].x, r.y);
+    }
+    // v[q] and v[R - q] are no longer read: every pair is in t and d
+    v[q] = cadd(m, r);
+    v[R - q] = csub(m, r);
+  }
+  v[0] = sum;
 }
 
 // q = t / d, r = t mod d for 0 <= t < 2^22 and 1 <= d <= 2^14, through the
@@ -189,12 +246,12 @@ __device__ __forceinline__ void stage_r(const float2* __restrict__ a, float2* __
 #pragma unroll
       for (int r = 1; r < R; ++r) x[r] = cmul(x[r], tw[r * jm * twstep]);
     }
-    if (R == 2) bfly2(x);
-    else if (R == 4) bfly4(x);
-    else if (R == 8) bfly8(x);
-    else if (R == 3) bfly3(x);
-    else if (R == 5) bfly5(x);
-    else bfly_direct<R>(x, tw, n);
+    if constexpr (R == 2) bfly2(x);
+    else if constexpr (R == 4) bfly4(x);
+    else if constexpr (R == 8) bfly8(x);
+    else if constexpr (R == 3) bfly3(x);
+    else if constexpr (R == 5) bfly5(x);
+    else bfly_odd<R>(x);
     const int idxD = jq * Ns * R + jm;
 #pragma unroll
     for (int q = 0; q < R; ++q) dst[(idxD + q * Ns) * es] = x[q];
@@ -230,6 +287,14 @@ __device__ __forceinline__ void stage_generic(const float2* __restrict__ a, floa
   }
 }
 
+// The two largest radices in registers, out of line: inlined they cost the frame
+// kernels registers at every length (500^2 windows: rows 4% slower).
+static __device__ __noinline__ void stage_prime(const float2* a, float2* b, const float2* tw, int n,
+                                                int R, int Ns, int nvec, int vs, int es, bool vfast) {
+  if (R == 11) stage_r<11>(a, b, tw, n, Ns, nvec, vs, es, vfast);
+  else stage_r<13>(a, b, tw, n, Ns, nvec, vs, es, vfast);
+}
+
 // The Stockham stages of a length-n transform with the given radices.
 __device__ inline float2* fft_stages(float2* a, float2* b, const int* radix, int nstages,
                                      const float2* tw, int n, int nvec, int vs, int es,
@@ -244,6 +309,8 @@ __device__ inline float2* fft_stages(float2* a, float2* b, const int* radix, int
       case 5: stage_r<5>(a, b, tw, n, Ns, nvec, vs, es, vfast); break;
       case 7: stage_r<7>(a, b, tw, n, Ns, nvec, vs, es, vfast); break;
       case 8: stage_r<8>(a, b, tw, n, Ns, nvec, vs, es, vfast); break;
+      case 11:
+      case 13: stage_prime(a, b, tw, n, R, Ns, nvec, vs, es, vfast); break;
       default: stage_generic(a, b, tw, n, R, Ns, nvec, vs, es); break;
     }
     __syncthreads();

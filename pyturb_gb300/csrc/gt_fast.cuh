@@ -62,11 +62,11 @@ __device__ __forceinline__ void gt_combine3(float2 (&x)[3][8]) {
 }
 
 // ------------------------------------------------------------------ rows
-// Generate (noise x filter) or plain complex rows; ROW_NV rows per CTA.
+// Generate (noise x filter) or plain complex rows, in place if `in` is `work`;
+// ROW_NV rows per CTA.
 template <int R1, int M>
 __global__ void __launch_bounds__(GtCfg<R1, M>::ROW_THREADS)
-k_rows_gt(const float2* __restrict__ tw, const float2* __restrict__ in, int gen, GenRowArgs ga,
-          float2* __restrict__ work) {
+k_rows_gt(const float2* __restrict__ tw, const float2* in, int gen, GenRowArgs ga, float2* work) {
   using G = GtCfg<R1, M>;
   constexpr int N = G::N, T = G::T, NV = G::ROW_NV, PAD = G::PAD, H = G::H;
   extern __shared__ float2 sm[];

@@ -48,6 +48,7 @@ namespace pt {
 
 constexpr int kMaxLevels = 16;
 constexpr int kThreads = 256;
+constexpr int kColThreads = 512;  // shared-memory column passes
 // Largest P * ns (float2) of first basis rows the column kernels stage in
 // shared memory for the subharmonic epilogue.
 constexpr int kColBasisMax = 4096;
@@ -68,12 +69,24 @@ static inline int gen_chunk(int ns) {
   size_t c = (size_t)(64u << 20) / per;
   return (int)std::max<size_t>(1, std::min<size_t>(256, c));
 }
-// Rows per CTA of the shared-memory row pass: about 2048 elements, so every
-// stage gives most of the 256 threads a butterfly.
-// rows / columns a CTA of the shared-memory passes transforms, from the
-// buffer length (fft_buf_len: M for a Bluestein grid)
-static inline int rows_per_cta(int nb) { return std::max(1, std::min(16, 2048 / nb)); }
+// Rows / columns a CTA of the shared-memory passes transforms, from the buffer
+// length (fft_buf_len: M for a Bluestein grid): about 4096 elements a CTA, so that
+// the stages of the larger radices still give most threads a butterfly. Rows of
+// three 728^2 images: 25.4 us at 2048 elements, 20.4 us so.
+static inline int rows_per_cta(int nb) { return std::max(1, std::min(16, 4096 / nb)); }
 static inline int cols_per_cta(int nb) { return std::max(1, std::min(16, 4096 / nb)); }
+// The shape of a column pass over `nimg` images: where such CTAs would not fill
+// the SMs three times over, more columns and threads a CTA (three 728^2 images:
+// 41.4 us at 4096 elements and 256 threads, 34.2 us at 6144 and 512; vectors of
+// fewer than 320 elements measured slower so, 278^2: 55.5 us against 59.0 us).
+struct ColShape {
+  int C, threads;
+};
+static inline ColShape col_shape(int ns, int nb, int nimg) {
+  const int C = cols_per_cta(nb);
+  if (nb < 320 || (long long)((ns + C - 1) / C) * nimg >= 3 * 152) return {C, kThreads};
+  return {std::max(1, std::min(16, 6144 / nb)), kColThreads};
+}
 
 static inline void count_launch(int k = 1) {
   __atomic_add_fetch(launch_counter(), (uint64_t)k, __ATOMIC_RELAXED);
@@ -174,11 +187,12 @@ __device__ __forceinline__ void gen_coef_pair(const GenRowArgs& a, int img) {
   gen_coef_warp(a, gc, w == 0 ? img : a.ch + img, lane);
 }
 
-// Plain complex rows (pt_ifft2) and generate rows share this kernel: `gen`
-// selects the producer. rpc rows per CTA, one transform per row.
+// Plain complex rows (pt_ifft2; frames, in place) and generate rows share this
+// kernel: `gen` selects the producer. rpc rows per CTA, one transform per row; a
+// CTA has read its rows before it writes them, so `in` may be `work`.
 __global__ void __launch_bounds__(kThreads)
-k_rows(FftDesc d, const float2* __restrict__ tw, int rpc, const float2* __restrict__ in,
-       int gen, GenRowArgs ga, float2* __restrict__ work) {
+k_rows(FftDesc d, const float2* __restrict__ tw, int rpc, const float2* in,
+       int gen, GenRowArgs ga, float2* work) {
   extern __shared__ float2 sm[];
   const int ns = d.n;
   const int row0 = blockIdx.x * rpc;
@@ -446,7 +460,8 @@ __device__ __forceinline__ float img_scale_of(const PairStore& st, int img) {
   return st.img_scale ? st.scale * __ldg(st.img_scale + img) : st.scale;
 }
 
-__global__ void __launch_bounds__(kThreads)
+template <int THREADS>
+__global__ void __launch_bounds__(THREADS)
 k_pair_cols(FftDesc d, const float2* __restrict__ tw, const float2* __restrict__ work, int C,
             int pair0, PairStore st) {
   extern __shared__ float2 sm[];
@@ -909,6 +924,102 @@ k_lgs_zoom_tile(int L, int ns, int n, const int32_t* __restrict__ idx, const flo
 #include "frames_fast.cuh"  // power-of-two fast path kernels
 #include "cols_tma.cuh"     // TMA-fed column pass
 #include "gt_fast.cuh"       // register transforms of length 3 * 2^k (Good-Thomas)
+#include "blu_fast.cuh"      // register Bluestein transforms
+
+// Layer sums of frames at arbitrary shifts on grids that are not a power of two:
+// Y[pair][kx][ky] = H_f0 + i H_f1 for every row, to be transformed in place by
+// the row pass of the grid's form. A thread owns one column ky and RB row pairs
+// {kx, -kx} of NF frames, so a phasor of the column serves RB rows and a value of
+// the spectra NF frames; the phasors are made here, from the exact fixed-point
+// phases. As in k_frame_rows_reg a layer costs one product an element and frame,
+// both products only on the Nyquist row and column of an even grid, and the CTAs
+// of the last block row make the subharmonic coefficients. Five frames of 9
+// layers on 728^2 took 81.6 us for coefficients, phasor tables and rows in one
+// shared-memory kernel, 44.3 us in this one and the row pass.
+constexpr int kSumThreads = 128;
+template <int NF, int RB, int CAP>
+__global__ void __launch_bounds__(kSumThreads)
+k_frame_sum(int n, const float2* __restrict__ spectra, const __grid_constant__ FramePrepArgs a,
+            const __grid_constant__ FrameShifts<CAP> sh, int fbeg, int nf, float2* __restrict__ work) {
+  extern __shared__ float2 pxs[];  // (NF, J, RB) row phasors
+  const int f0 = NF * blockIdx.z;  // within this launch
+  const int live = min(NF, nf - f0);
+  const int J = a.J, rows = n / 2 + 1;
+  const FrameShift* fs = sh.v + f0 * J;
+  if ((int)blockIdx.y * RB >= rows) {  // subharmonic coefficients, a frame a CTA
+    if ((int)blockIdx.x < live) {
+      const FrameShift* q = fs + blockIdx.x * J;
+      frame_coef(a, fbeg + f0 + blockIdx.x, [&](int j, double& x, double& y) { x = q[j].sx; y = q[j].sy; });
+    }
+    return;
+  }
+  const int kx0 = blockIdx.y * RB;
+  for (int i = threadIdx.x; i < live * J * RB; i += kSumThreads) {
+    const int r = i % RB, fj = i / RB;
+    pxs[i] = phasor_from_fixed((uint64_t)(int64_t)signed_freq(min(kx0 + r, rows - 1), n) * fs[fj].ux);
+  }
+  __syncthreads();
+  const int ky = blockIdx.x * kSumThreads + threadIdx.x;
+  if (ky >= n) return;
+  const int nky = ky == 0 ? 0 : n - ky;
+  const bool even = (n & 1) == 0, nyq_col = even && ky == n / 2;
+  const uint64_t kys = (uint64_t)(int64_t)signed_freq(ky, n);
+  const size_t plane = (size_t)n * n;
+  float2 h[NF][RB];
+#pragma unroll
+  for (int f = 0; f < NF; ++f)
+#pragma unroll
+    for (int r = 0; r < RB; ++r) h[f][r] = make_float2(0.f, 0.f);
+  auto load = [&](int l, float2 (&s)[RB], float2 (&t)[RB]) {
+    const float2* sl = spectra + (size_t)l * plane;
+#pragma unroll
+    for (int r = 0; r < RB; ++r) {
+      const int kx = min(kx0 + r, rows - 1), nkx = kx == 0 ? 0 : n - kx;
+      s[r] = __ldg(sl + (size_t)kx * n + ky);
+      t[r] = __ldg(sl + (size_t)nkx * n + nky);
+    }
+  };
+  auto add = [&](int f, int j, const float2 (&s)[RB], const float2 (&t)[RB]) {
+    const float2 py = phasor_from_fixed(kys * fs[f * J + j].uy);
+    const float2* px = pxs + (size_t)(f * J + j) * RB;
+#pragma unroll
+    for (int r = 0; r < RB; ++r) {
+      const bool nyq_row = even && kx0 + r == n / 2;
+      if (nyq_row || nyq_col) {
+        const float2 qc = cmul(nyq_row ? cconj(px[r]) : px[r], nyq_col ? cconj(py) : py);
+        const float2 x = cfma(s[r], cmul(px[r], py), cmul(cconj(t[r]), qc));
+        h[f][r] = cadd(h[f][r], cscale(x, 0.5f));
+      } else {
+        const float2 m = make_float2(0.5f * (s[r].x + t[r].x), 0.5f * (s[r].y - t[r].y));
+        h[f][r] = cfma(m, cmul(px[r], py), h[f][r]);
+      }
+    }
+  };
+  for (int j = 0; j < J; ++j) {
+    float2 s[RB], t[RB];
+    if (!a.per_layer) load(j, s, t);
+#pragma unroll
+    for (int f = 0; f < NF; ++f) {
+      if (f >= live) break;
+      if (a.per_layer) load(a.frame0 + fbeg + f0 + f, s, t);
+      add(f, j, s, t);
+    }
+  }
+#pragma unroll
+  for (int f = 0; f < NF; f += 2) {
+    if (f >= live) break;
+    float2* img = work + (size_t)((fbeg + f0 + f) / 2) * plane;
+#pragma unroll
+    for (int r = 0; r < RB; ++r) {
+      const int kx = kx0 + r;
+      if (kx >= rows) break;
+      const float2 p = h[f][r], q = h[f + 1][r];
+      img[(size_t)kx * n + ky] = make_float2(p.x - q.y, p.y + q.x);
+      if (kx != 0 && 2 * kx != n)  // Y(-k) = conj H0(k) + i conj H1(k)
+        img[(size_t)(n - kx) * n + nky] = make_float2(p.x + q.y, q.x - p.y);
+    }
+  }
+}
 
 // ================================================================ host helpers
 // shared memory of the generic passes: nb = fft_buf_len of the grid's
@@ -1115,6 +1226,16 @@ static int launch_uniform_reg_chunk(const pt_grid* g, const float2* spectra, con
   return uniform_reg_rows_t<16>(g, spectra, L, nf, ut, w.hn, w.img, s);
 }
 
+// shifts of global frames [f0, f0 + nf), term by term
+static void fill_shifts(FrameShift* v, const FramePrepArgs& pa, const double* sx, const double* sy,
+                        int f0, int nf) {
+  for (int f = 0; f < nf; ++f)
+    for (int j = 0; j < pa.J; ++j) {
+      const size_t src = pa.per_layer ? (size_t)f0 + f : ((size_t)f0 + f) * pa.J + j;
+      v[f * pa.J + j] = FrameShift{sx[src], sy[src], host_fixed(sx[src] * pa.df), host_fixed(sy[src] * pa.df)};
+    }
+}
+
 // ---- frames at arbitrary shifts on power-of-two grids
 static bool frames_reg(int ns, int J) {
   return ns >= 128 && ns <= 2048 && (ns & (ns - 1)) == 0 && 2 * J <= kShiftTermsMany;
@@ -1132,13 +1253,7 @@ static int frame_rows_reg_t(const pt_grid* g, const float2* spectra, const Frame
   for (int fb = 0; fb < pa.F; fb += fsub) {
     const int nf = std::min(fsub, pa.F - fb);
     FrameShifts<CAP> sh;
-    for (int f = 0; f < nf; ++f)
-      for (int j = 0; j < pa.J; ++j) {
-        const size_t gf = (size_t)f0 + fb + f;
-        const size_t src = pa.per_layer ? gf : gf * pa.J + j;
-        sh.v[f * pa.J + j] = FrameShift{sx[src], sy[src], host_fixed(sx[src] * pa.df),
-                                        host_fixed(sy[src] * pa.df)};
-      }
+    fill_shifts(sh.v, pa, sx, sy, f0 + fb, nf);
     ProfScope ps("k_frame_rows", s);
     kern<<<dim3(N / 2 + 1 + (pa.P > 0), (nf + 1) / 2), Cfg::THREADS, smem, s>>>(g->tw, spectra, pa,
                                                                                sh, fb, nf, img);
@@ -1161,6 +1276,40 @@ static int launch_frame_rows_reg(const pt_grid* g, const float2* spectra, const 
 #undef PT_CASE
   }
   return fail(PT_ERR_UNSUPPORTED, "frame_rows_reg: not an instantiated size");
+}
+
+// ---- frames at arbitrary shifts on other grids
+static bool frames_sum(int ns, int J) { return (ns & (ns - 1)) != 0 && 4 * J <= kShiftTermsMany; }
+
+template <int NF, int CAP>
+static int frame_sum_t(const pt_grid* g, const float2* spectra, const FramePrepArgs& pa,
+                       const double* sx, const double* sy, int f0, float2* img, cudaStream_t s) {
+  constexpr int RB = 4;
+  const int n = g->ns;
+  auto kern = k_frame_sum<NF, RB, CAP>;
+  const size_t smem = (size_t)NF * pa.J * RB * sizeof(float2);
+  const int fsub = CAP / pa.J / NF * NF;  // frames a launch takes
+  for (int fb = 0; fb < pa.F; fb += fsub) {
+    const int nf = std::min(fsub, pa.F - fb);
+    FrameShifts<CAP> sh;
+    fill_shifts(sh.v, pa, sx, sy, f0 + fb, nf);
+    ProfScope ps("k_frame_sum", s);
+    const int cols = (n + kSumThreads - 1) / kSumThreads, rows = (n / 2 + RB) / RB;
+    kern<<<dim3(std::max(cols, pa.P > 0 ? NF : 0), rows + (pa.P > 0), (nf + NF - 1) / NF), kSumThreads, smem,
+           s>>>(n, spectra, pa, sh, fb, nf, img);
+    count_launch();
+  }
+  return PT_OK;
+}
+static int launch_frame_sum(const pt_grid* g, const float2* spectra, const FramePrepArgs& pa,
+                            const double* sx, const double* sy, int f0, float2* img, cudaStream_t s) {
+  // four frames to a pass over the spectra, but no more than there are
+  const bool few = (pa.F + 3) / 4 * 4 * pa.J <= kShiftTermsFew;
+  if (pa.F <= 2)
+    return few ? frame_sum_t<2, kShiftTermsFew>(g, spectra, pa, sx, sy, f0, img, s)
+               : frame_sum_t<2, kShiftTermsMany>(g, spectra, pa, sx, sy, f0, img, s);
+  return few ? frame_sum_t<4, kShiftTermsFew>(g, spectra, pa, sx, sy, f0, img, s)
+             : frame_sum_t<4, kShiftTermsMany>(g, spectra, pa, sx, sy, f0, img, s);
 }
 
 // ---- power-of-two dispatch (runtime ns -> template N)
@@ -1355,6 +1504,77 @@ static int pair_cols_gt(const pt_grid* g, const float2* work, int npair, int pai
     case 512: return pair_cols_gt_t<512>(g, work, npair, pair0, st, s);
   }
   return fail(PT_ERR_UNSUPPORTED, "pair_cols_gt: not 3 x 2^k");
+}
+
+// A launch that is a programmatic dependent of the one before it on the stream:
+// its CTAs stage their twiddles while that one's last wave runs, then wait for it
+// (griddepcontrol.wait).
+template <class... KArgs, class... Args>
+static int launch_dependent(const char* name, void (*kern)(KArgs...), dim3 grid, int threads,
+                            size_t smem, cudaStream_t s, Args... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return check_cuda(cudaLaunchKernelEx(&cfg, kern, args...), name);
+}
+
+// ---- register Bluestein path
+template <int M>
+static int rows_blu_t(const FftDesc& d, const float2* in, int gen, const GenRowArgs& ga, int nimg,
+                      float2* work, cudaStream_t s) {
+  using Cfg = BluCfg<M>;
+  const size_t smem = (size_t)(M + 2 * Cfg::NV * fft_padded(M)) * sizeof(float2);
+  if (int rc = set_smem(k_rows_blu<M>, smem, "k_rows_blu")) return rc;
+  ProfScope ps("k_rows", s);
+  const int per = Cfg::NV * Cfg::RPT;
+  k_rows_blu<M><<<dim3((d.n + per - 1) / per, nimg), Cfg::THREADS, smem, s>>>(d, in, gen, ga, work);
+  return PT_OK;
+}
+template <int M>
+static int cols_blu_t(const pt_grid* g, const FftDesc& d, const float2* work, int nimg, int pair0,
+                      const PairStore* st, float2* out, cudaStream_t s) {
+  using Cfg = BluCfg<M>;
+  const dim3 grid((d.n + Cfg::C - 1) / Cfg::C, nimg);
+  const size_t smem = (size_t)(M + 2 * M * Cfg::C + (st ? 8 * g->P * Cfg::C : 0)) * sizeof(float2);
+  ProfScope ps(st ? "k_pair_cols" : "k_plain_cols", s);
+  if (st) {
+    if (int rc = set_smem(k_pair_cols_blu<M>, smem, "k_pair_cols_blu")) return rc;
+    return launch_dependent("k_pair_cols_blu", k_pair_cols_blu<M>, grid, Cfg::COL_THREADS, smem, s, d,
+                            work, pair0, *st);
+  }
+  if (int rc = set_smem(k_plain_cols_blu<M>, smem, "k_plain_cols_blu")) return rc;
+  return launch_dependent("k_plain_cols_blu", k_plain_cols_blu<M>, grid, Cfg::COL_THREADS, smem, s, d,
+                          work, out);
+}
+static int rows_blu(const FftDesc& d, const float2* in, int gen, const GenRowArgs& ga, int nimg,
+                    float2* work, cudaStream_t s) {
+  switch (d.M) {
+    case 256: return rows_blu_t<256>(d, in, gen, ga, nimg, work, s);
+    case 512: return rows_blu_t<512>(d, in, gen, ga, nimg, work, s);
+    case 1024: return rows_blu_t<1024>(d, in, gen, ga, nimg, work, s);
+    case 2048: return rows_blu_t<2048>(d, in, gen, ga, nimg, work, s);
+    case 4096: return rows_blu_t<4096>(d, in, gen, ga, nimg, work, s);
+  }
+  return fail(PT_ERR_UNSUPPORTED, "rows_blu: padded length not instantiated");
+}
+// `st`: the paired epilogue; else plain columns to out
+static int cols_blu(const pt_grid* g, const FftDesc& d, const float2* work, int nimg, int pair0,
+                    const PairStore* st, float2* out, cudaStream_t s) {
+  switch (d.M) {
+    case 256: return cols_blu_t<256>(g, d, work, nimg, pair0, st, out, s);
+    case 512: return cols_blu_t<512>(g, d, work, nimg, pair0, st, out, s);
+    case 1024: return cols_blu_t<1024>(g, d, work, nimg, pair0, st, out, s);
+    case 2048: return cols_blu_t<2048>(g, d, work, nimg, pair0, st, out, s);
+    case 4096: return cols_blu_t<4096>(g, d, work, nimg, pair0, st, out, s);
+  }
+  return fail(PT_ERR_UNSUPPORTED, "cols_blu: padded length not instantiated");
 }
 
 static int pair_cols_reg(const pt_grid* g, const float2* work, int npair, int pair0,
@@ -1623,7 +1843,8 @@ extern "C" int pt_ifft2(const pt_grid* g, const float* in, float* out, int batch
   const int ns = g->ns, blen = fft_buf_len(g->desc), ch = gen_chunk(ns),
             rpc = rows_per_cta(blen), C = cols_per_cta(blen);
   const size_t rs = rows_smem(ns, blen, rpc), cs = cols_smem(ns, blen, C, 0);
-  if (!pow2_fast(ns)) {
+  const bool blu = blu_fast(g->desc);
+  if (!pow2_fast(ns) && !blu) {
     if (int rc = set_smem(k_rows, rs, "k_rows")) return rc;
     if (int rc = set_smem(k_plain_cols, cs, "k_plain_cols")) return rc;
   }
@@ -1635,6 +1856,9 @@ extern "C" int pt_ifft2(const pt_grid* g, const float* in, float* out, int batch
     if (pow2_fast(ns)) {
       if (int rc = rows_reg(g, src, 0, none, nb, w.img, s)) return rc;
       if (int rc = plain_cols_reg(g, w.img, nb, dst, s)) return rc;
+    } else if (blu) {
+      if (int rc = rows_blu(g->desc, src, 0, none, nb, w.img, s)) return rc;
+      if (int rc = cols_blu(g, g->desc, w.img, nb, 0, nullptr, dst, s)) return rc;
     } else {
       {
         ProfScope ps("k_rows", s);
@@ -1669,9 +1893,10 @@ static int generate_impl(const pt_grid* g, int count, const float* amplitude,
   const int blen = fft_buf_len(g->desc);
   const int ch = gen_chunk(ns), rpc = rows_per_cta(blen), C = cols_per_cta(blen);
   const size_t rs = rows_smem(ns, blen, rpc), cs = cols_smem(ns, blen, C, P);
-  if (!pow2_fast(ns) && !gt_m(ns)) {
+  const bool blu = blu_fast(g->desc);
+  if (!pow2_fast(ns) && !gt_m(ns) && !blu) {
     if (int rc = set_smem(k_rows, rs, "k_rows")) return rc;
-    if (int rc = set_smem(k_pair_cols, cs, "k_pair_cols")) return rc;
+    if (int rc = set_smem(k_pair_cols<kThreads>, cs, "k_pair_cols")) return rc;
   }
   for (int b0 = 0; b0 < n_fft; b0 += ch) {
     const int nb = std::min(ch, n_fft - b0);
@@ -1681,6 +1906,8 @@ static int generate_impl(const pt_grid* g, int count, const float* amplitude,
       if (int rc = rows_reg(g, nullptr, 1, ga, nb, w.img, s)) return rc;
     } else if (gt_m(ns)) {
       if (int rc = rows_gt(g, nullptr, 1, ga, nb, w.img, s)) return rc;
+    } else if (blu) {
+      if (int rc = rows_blu(g->desc, nullptr, 1, ga, nb, w.img, s)) return rc;
     } else {
       ProfScope ps("k_rows", s);
       k_rows<<<dim3((ns + rpc - 1) / rpc, nb), kThreads, rs, s>>>(g->desc, g->tw, rpc, nullptr, 1,
@@ -1711,9 +1938,11 @@ static int generate_impl(const pt_grid* g, int count, const float* amplitude,
       if (int rc = pair_cols_reg(g, w.img, nb, b0, st, s)) return rc;
     } else if (gt_m(ns)) {
       if (int rc = pair_cols_gt(g, w.img, nb, b0, st, s)) return rc;
+    } else if (blu) {
+      if (int rc = cols_blu(g, g->desc, w.img, nb, b0, &st, nullptr, s)) return rc;
     } else {
       ProfScope ps("k_pair_cols", s);
-      k_pair_cols<<<dim3((ns + C - 1) / C, nb), kThreads, cs, s>>>(g->desc, g->tw, w.img, C, b0, st);
+      k_pair_cols<kThreads><<<dim3((ns + C - 1) / C, nb), kThreads, cs, s>>>(g->desc, g->tw, w.img, C, b0, st);
     }
     count_launch();
     if (int rc = check_launch("pt_generate")) return rc;
@@ -1783,12 +2012,11 @@ extern "C" int pt_frames(const pt_grid* g, int L, const float* spectra, const fl
   cudaStream_t s = (cudaStream_t)stream;
   const FftDesc fd = frame_desc(g);
   const int blen = fft_buf_len(fd);
-  const int ch = image_chunk(ns), C = cols_per_cta(blen);
+  const int ch = image_chunk(ns);
   const int J = per_layer ? 1 : L;
   if (2 * J > kShiftDoubles) return fail(PT_ERR_UNSUPPORTED, "pt_frames: at most 896 layers");
-  const size_t rs = frame_rows_smem(ns, blen), cs = cols_smem(ns, blen, C, P);
-  if (!pow2_fast(ns))
-    if (int rc = set_smem(k_pair_cols, cs, "k_pair_cols")) return rc;
+  const size_t rs = frame_rows_smem(ns, blen);
+  const bool blu = blu_fast(g->desc);
   const int fchunk = 2 * ch;
   const int fsub = std::max(1, kShiftDoubles / (2 * J));  // frames per parameter block
   for (int f0 = 0; f0 < F; f0 += fchunk) {
@@ -1818,13 +2046,30 @@ extern "C" int pt_frames(const pt_grid* g, int L, const float* spectra, const fl
                                             sx, sy, f0, nf, w, s))
         return rc;
     }
-    const bool reg = !uni && frames_reg(ns, J);
+    const bool reg = !uni && frames_reg(ns, J), sum = !uni && !reg && frames_sum(ns, J);
     if (reg) {
       // phasors, layer sums, row transforms and coefficients in one launch
       if (int rc = launch_frame_rows_reg(g, (const float2*)spectra, pa, sx, sy, f0, w.img, s))
         return rc;
     }
-    for (int fb = 0; fb < nf && !uni_reg && !reg; fb += fsub) {
+    if (sum) {
+      // phasors, layer sums and coefficients, then the grid's own row pass in place
+      if (int rc = launch_frame_sum(g, (const float2*)spectra, pa, sx, sy, f0, w.img, s)) return rc;
+      const GenRowArgs none{};
+      if (blu) {
+        if (int rc = rows_blu(g->desc, w.img, 0, none, npair, w.img, s)) return rc;
+      } else if (gt_m(ns)) {
+        if (int rc = rows_gt(g, w.img, 0, none, npair, w.img, s)) return rc;
+      } else {
+        const int rb = fft_buf_len(g->desc), rpc = rows_per_cta(rb);
+        const size_t rsm = rows_smem(ns, rb, rpc);
+        if (int rc = set_smem(k_rows, rsm, "k_rows")) return rc;
+        ProfScope ps("k_rows", s);
+        k_rows<<<dim3((ns + rpc - 1) / rpc, npair), kThreads, rsm, s>>>(g->desc, g->tw, rpc, w.img, 0,
+                                                                       none, w.img);
+      }
+    }
+    for (int fb = 0; fb < nf && !uni_reg && !reg && !sum; fb += fsub) {
       const int nb = std::min(fsub, nf - fb);
       ShiftParams sp;
       for (int f = 0; f < nb; ++f)
@@ -1843,7 +2088,7 @@ extern "C" int pt_frames(const pt_grid* g, int L, const float* spectra, const fl
       k_frame_phasors<<<dim3((ns + 255) / 256, nb * J), 256, 0, s>>>(pa, sp, fb);
       count_launch();
     }
-    if (uni_reg || reg) {
+    if (uni_reg || reg || sum) {
       // rows done above
     } else if (uni) {
       if (int rc = launch_uniform_rows(g, (const float2*)spectra, L, sx, sy, f0, nf, w.hn, w.px,
@@ -1877,10 +2122,22 @@ extern "C" int pt_frames(const pt_grid* g, int L, const float* spectra, const fl
     st.sym = g->sym;
     if (pow2_fast(ns)) {
       if (int rc = pair_cols_reg(g, w.img, npair, 0, st, s)) return rc;
+    } else if (gt_m(ns)) {
+      if (int rc = pair_cols_gt(g, w.img, npair, 0, st, s)) return rc;
+    } else if (blu) {
+      if (int rc = cols_blu(g, g->desc, w.img, npair, 0, &st, nullptr, s)) return rc;
     } else {
       ProfScope ps("k_pair_cols", s);
-      k_pair_cols<<<dim3((ns + C - 1) / C, npair), kThreads, cs, s>>>(fd, g->tw, w.img, C, 0,
-                                                                     st);
+      const ColShape sh = col_shape(ns, blen, npair);
+      const size_t csm = cols_smem(ns, blen, sh.C, P);
+      const dim3 grid((ns + sh.C - 1) / sh.C, npair);
+      if (sh.threads == kThreads) {
+        if (int rc = set_smem(k_pair_cols<kThreads>, csm, "k_pair_cols")) return rc;
+        k_pair_cols<kThreads><<<grid, kThreads, csm, s>>>(fd, g->tw, w.img, sh.C, 0, st);
+      } else {
+        if (int rc = set_smem(k_pair_cols<kColThreads>, csm, "k_pair_cols")) return rc;
+        k_pair_cols<kColThreads><<<grid, kColThreads, csm, s>>>(fd, g->tw, w.img, sh.C, 0, st);
+      }
     }
     count_launch();
     if (int rc = check_launch("pt_frames")) return rc;
