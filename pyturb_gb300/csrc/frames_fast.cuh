@@ -304,6 +304,155 @@ k_pair_cols_reg(const float2* __restrict__ tw, const float2* __restrict__ work, 
   }
 }
 
+// The same pass as a persistent, software-pipelined kernel (N = 256, 512, 1024,
+// symmetric subharmonic bases): a CTA walks (column tile, pair) items; while the
+// epilogue of one item computes and stores, the next item's tile, coefficients
+// and means are on their way to shared memory by cp.async, and the twiddles and
+// the first basis row of each level are staged once a CTA instead of once a tile.
+// The tile's buffer is also the transform's second exchange buffer: the first
+// exchange's barrier comes after every thread has taken its inputs from it. The
+// one-tile-a-CTA kernel above waits a load latency three times a tile with the SM
+// to itself. 32 pairs of 512^2: 51.4 us in that form, 40.3 us so with 16 columns a
+// CTA, 41 us with 8 and two CTAs an SM, which leaves short frame windows 5% less
+// (4-layer windows of 512^2: 1116 and 1065 us a thousand frames; 1334 us before).
+template <int N>
+struct PipeCfg {
+  static constexpr int C = 8;
+  static constexpr int T = N / 8;
+  static constexpr int THREADS = C * T;
+  static constexpr int PER_SM = 1024 / THREADS;  // 64 registers a thread
+};
+template <int N>
+static size_t pipe_smem(int P) {
+  constexpr int C = PipeCfg<N>::C;
+  // twiddles, exchange buffer, tile, basis rows, (U, W) of both screens, K, coefficients, means
+  return ((size_t)N + 2 * N * C + (size_t)P * N + 2 * P * C + P * C + 18 * P + 1) * sizeof(float2);
+}
+__device__ __forceinline__ void cp_async(void* dst, const void* src, int bytes) {
+  const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst);
+  if (bytes == 16) asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d), "l"(src) : "memory");
+  else if (bytes == 8) asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(d), "l"(src) : "memory");
+  else asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(d), "l"(src) : "memory");
+}
+
+template <int N>
+__global__ void __launch_bounds__(PipeCfg<N>::THREADS, PipeCfg<N>::PER_SM)
+k_pair_cols_pipe(const float2* __restrict__ tw, const float2* work, int npair, int pair0,
+                 const __grid_constant__ PairStore st) {
+  using Cfg = PipeCfg<N>;
+  constexpr int T = Cfg::T, C = Cfg::C, THREADS = Cfg::THREADS, NT = N / C;
+  extern __shared__ __align__(16) float2 sm[];
+  const int P = st.P;
+  float2* stw = sm;
+  float2* ebuf = sm + N;                 // first exchange
+  float2* tile = ebuf + N * C;           // (N, C) input, then the second exchange
+  float2* sbasis = tile + N * C;         // (P, N)
+  float4* utab = (float4*)(sbasis + P * N);  // (P, C): U_re, W_re, U_im, W_im
+  float2* ktab = (float2*)(utab + P * C);    // (P, C): K_re, K_im of each level
+  float2* scoef = ktab + P * C;          // (2, P, 9)
+  float* smean = (float*)(scoef + 18 * P);  // (2)
+  const int tid = threadIdx.x, c = tid % C, j = tid / C;
+  const ColLayout<C> se{ebuf + c}, st2{tile + c};
+  load_stage_tw<N>(stw, tw);
+  for (int i = tid; i < P * N; i += THREADS)
+    sbasis[i] = __ldg(st.basis + (size_t)(3 * (i / N)) * N + (i % N));
+  // launched as a programmatic dependent of the row pass: everything below
+  // reads what that pass wrote
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  const int items = NT * npair;
+  auto fetch = [&](int item) {
+    const int pl = item / NT, y0 = item % NT * C, pair = pair0 + pl;
+    const float2* src = work + (size_t)pl * N * N + y0;
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {  // 16-byte pieces: two columns of a row
+      const int e = tid + q * THREADS, r = e / (C / 2), h = e % (C / 2);
+      cp_async(tile + r * C + 2 * h, src + (size_t)r * N + 2 * h, 16);
+    }
+    for (int e = tid; e < 18 * P; e += THREADS) {
+      const int o = e / (9 * P), k = e - o * 9 * P;
+      const bool live = pair * (o ? st.im_mul : st.re_mul) + (o ? st.im_add : st.re_add) < st.count;
+      const int row = pl * st.crow_mul + (o ? st.crow_im : st.crow_re);
+      if (live) {
+        cp_async(scoef + e, st.coef + (size_t)row * 9 * P + k, 8);
+        if (k == 0) cp_async(smean + o, st.mean + row, 4);
+      }
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  if ((int)blockIdx.x < items) fetch(blockIdx.x);
+  const bool full = st.crop == 0 && st.n_out == N;  // every row of a column is kept
+  const size_t plane = (size_t)st.n_out * st.n_out;
+  for (int item = blockIdx.x; item < items; item += gridDim.x) {
+    const int y = item % NT * C + c, pair = pair0 + item / NT;
+    const int img_re = pair * st.re_mul + st.re_add, img_im = pair * st.im_mul + st.im_add;
+    const bool do_re = img_re < st.count, do_im = img_im < st.count;
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    __syncthreads();
+    float2 x[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) x[i] = tile[(j + T * i) * C + c];
+    // the column tables of this item (a thread a level, screen and column), read
+    // after the transform's barriers: m_i = sum_j coef_ij b_j(y), b = (b0, 1, conj b0)
+    for (int q = tid; q < 2 * P * C; q += THREADS) {
+      const int cc = q % C, p = q / C % P, o = q / (C * P);
+      const float2 b = sbasis[p * N + item % NT * C + cc];
+      const float2* cf = scoef + o * 9 * P + 9 * p;
+      float2 m[3];
+#pragma unroll
+      for (int i = 0; i < 3; ++i)
+        m[i] = cfma(cf[3 * i + 2], cconj(b), cadd(cf[3 * i + 1], cmul(cf[3 * i], b)));
+      float* u = (float*)(utab + p * C + cc) + 2 * o;
+      u[0] = m[0].x + m[2].x;
+      u[1] = m[2].y - m[0].y;
+      ((float*)(ktab + p * C + cc))[o] = m[1].x;
+    }
+    reg_fft_db<N>(x, j, stw, se, st2);
+    const float mre = P > 0 && do_re ? smean[0] : 0.f, mim = P > 0 && do_im ? smean[1] : 0.f;
+    __syncthreads();  // the tile and the coefficients are spent
+    if (item + (int)gridDim.x < items) fetch(item + gridDim.x);
+    const int yo = y - st.crop;
+    if (yo < 0 || yo >= st.n_out) continue;
+    float k0 = 0.f, k1 = 0.f;
+    for (int p = 0; p < P; ++p) {
+      const float2 k = ktab[p * C + c];
+      k0 += k.x;
+      k1 += k.y;
+    }
+    k0 -= mre;
+    k1 -= mim;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      x[i].x += k0;
+      x[i].y += k1;
+    }
+    for (int p = 0; p < P; ++p) {
+      const float4 u = utab[p * C + c];
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        const float2 b = sbasis[p * N + j + T * i];
+        x[i].x = fmaf(b.x, u.x, fmaf(b.y, u.y, x[i].x));
+        x[i].y = fmaf(b.x, u.z, fmaf(b.y, u.w, x[i].y));
+      }
+    }
+    const float sre = do_re ? img_scale_of(st, img_re) : 0.f, sim = do_im ? img_scale_of(st, img_im) : 0.f;
+    float* ore = st.out + (size_t)(do_re ? img_re : 0) * plane + yo;
+    float* oim = st.out + (size_t)(do_im ? img_im : 0) * plane + yo;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const int xo = j + T * i - st.crop;
+      if (!full && (xo < 0 || xo >= st.n_out)) continue;
+      const size_t o = (size_t)xo * st.n_out;
+      if (st.accumulate) {
+        if (do_re) ore[o] += sre * x[i].x;
+        if (do_im) oim[o] += sim * x[i].y;
+      } else {
+        if (do_re) __stcs(ore + o, sre * x[i].x);
+        if (do_im) __stcs(oim + o, sim * x[i].y);
+      }
+    }
+  }
+}
+
 // ------------------------------------------------------------------ uniform frames
 // Fused synthesis + row transform. CTA = the row pair {kx, N - kx} of one
 // anchor block of frames. Threads first own columns (E each) and advance the

@@ -1577,8 +1577,31 @@ static int cols_blu(const pt_grid* g, const FftDesc& d, const float2* work, int 
   return fail(PT_ERR_UNSUPPORTED, "cols_blu: padded length not instantiated");
 }
 
+template <int N>
+static int pair_cols_pipe_t(const pt_grid* g, const float2* work, int npair, int pair0,
+                            const PairStore& st, cudaStream_t s) {
+  using Cfg = PipeCfg<N>;
+  const size_t smem = pipe_smem<N>(g->P);
+  if (int rc = set_smem(k_pair_cols_pipe<N>, smem, "k_pair_cols_pipe")) return rc;
+  ProfScope ps("k_pair_cols", s);
+  const int grid = std::min(N / Cfg::C * npair, 152 * Cfg::PER_SM);
+  return launch_dependent("k_pair_cols_pipe", k_pair_cols_pipe<N>, dim3(grid), Cfg::THREADS, smem, s,
+                          (const float2*)g->tw, work, npair, pair0, st);
+}
+// symmetric bases whose staged rows fit beside the tiles of two CTAs an SM (one at
+// 1024), and images that 16-byte pieces can be fetched from
+static bool pair_cols_pipe(const pt_grid* g, const float2* work, const PairStore& st) {
+  return st.sym && g->P * g->ns <= kColBasisMax && ((uintptr_t)work & 15) == 0 &&
+         (g->ns == 256 || g->ns == 512 || g->ns == 1024);
+}
+
 static int pair_cols_reg(const pt_grid* g, const float2* work, int npair, int pair0,
                          const PairStore& st, cudaStream_t s) {
+  if (g->cols_variant == 0 && pair_cols_pipe(g, work, st)) {
+    if (g->ns == 256) return pair_cols_pipe_t<256>(g, work, npair, pair0, st, s);
+    if (g->ns == 512) return pair_cols_pipe_t<512>(g, work, npair, pair0, st, s);
+    return pair_cols_pipe_t<1024>(g, work, npair, pair0, st, s);
+  }
   if (g->cols_variant == 1) {
     if (g->ns == 256) return pair_cols_tma_t<256>(g, work, npair, pair0, st, s);
     if (g->ns == 512) return pair_cols_tma_t<512>(g, work, npair, pair0, st, s);
