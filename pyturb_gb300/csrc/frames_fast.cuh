@@ -671,7 +671,9 @@ struct UniformPrep {
   float2* hn;    // (F, 2N)
   float2* coef;  // (F, P, 9)
   float* mean;   // (F)
-  int N, L, P, F, nb;
+  float2* img;   // where the Nyquist cross goes as frame pairs instead of hn, or NULL
+  int N, L, P, F;
+  int nb, run;   // anchors and the frames between them
   int blocks_tab, blocks_nyq;
 };
 
@@ -685,7 +687,7 @@ __global__ void __launch_bounds__(256) k_uniform_prep(UniformPrep a) {
     const int b = bl / L, l = bl % L;
     const uint64_t kk = (uint64_t)(int64_t)signed_freq(k, N);
     if (b < a.nb) {
-      const uint64_t f0 = (uint64_t)b * kAnchor;
+      const uint64_t f0 = (uint64_t)b * a.run;
       a.px0[(size_t)bl * N + k] = phasor_from_fixed(kk * (a.up.ux0[l] + f0 * a.up.dux[l]));
       a.py0[(size_t)bl * N + k] = phasor_from_fixed(kk * (a.up.uy0[l] + f0 * a.up.duy[l]));
     } else {
@@ -736,6 +738,15 @@ __global__ void __launch_bounds__(256) k_uniform_prep(UniformPrep a) {
         x1 = cmul(x1, r1);
         x2 = cmul(x2, r2);
       }
+    }
+    if (a.img) {
+#pragma unroll
+      for (int f = 0; f < kNyqGroup; f += 2) {
+        if (f >= nfr) break;
+        const float2 h1 = f + 1 < nfr ? h[f + 1] : make_float2(0.f, 0.f);
+        a.img[((size_t)(fbeg + f) / 2 * N + kx) * N + ky] = make_float2(h[f].x - h1.y, h[f].y + h1.x);
+      }
+      return;
     }
 #pragma unroll
     for (int f = 0; f < kNyqGroup; ++f)

@@ -311,13 +311,10 @@ k_frame_rows(FftDesc d, const float2* __restrict__ tw, FrameRowArgs a, float2* _
 // so each thread keeps A_l = Sh_l Q_l R_l^f and R_l in registers and advances
 // a frame with one complex multiply-add per layer — no phasor tables. Anchors
 // (exact 64-bit fixed-point phases, u0 + f du mod 1) are re-taken every
-// kAnchor frames, bounding the float32 drift of the recurrence.
-// CTA = one row kx x kFramesPerCta frames; thread = one column ky; frame
-// pairs are packed as Y = H_f0 + i H_f1 and kPairsPerFft rows are transformed
-// together.
+// kAnchor frames at most, bounding the float32 drift of the recurrence. Frame
+// pairs are packed as Y = H_f0 + i H_f1.
 constexpr int kMaxUniformLayers = 16;
 constexpr int kAnchor = 64;
-constexpr int kPairsPerFft = 4;
 
 struct UniformParams {
   uint64_t ux0[kMaxUniformLayers], uy0[kMaxUniformLayers];  // frac(s0 df) of frame 0
@@ -330,110 +327,9 @@ __device__ __forceinline__ float2 phasor2(int kxs, int kys, uint64_t ux, uint64_
 
 // The phasor of the Nyquist index ns/2 is exp(-i pi ns u) on both k and -k
 // (fftfreq gives -ns/2 for it), so Q(-k) = conj Q(k) fails on the Nyquist
-// row and column and the shortcut through Sh does not hold there. This kernel
+// row and column and the shortcut through Sh does not hold there: the prep launch
 // forms H_f(k) = (X_f(k) + conj X_f(-k)) / 2 exactly on that cross (element e:
 // e < ns is (ns/2, e), else (e - ns, ns/2)) for every frame of the chunk.
-__global__ void k_nyquist_h(int ns, const float2* __restrict__ spectra, int L, int F,
-                            UniformParams up, float2* __restrict__ hn) {
-  const int e = blockIdx.x * blockDim.x + threadIdx.x;
-  const int f = blockIdx.y;
-  if (e >= 2 * ns || f >= F) return;
-  const int kx = e < ns ? ns / 2 : e - ns;
-  const int ky = e < ns ? e : ns / 2;
-  const int nkx = (ns - kx) % ns, nky = (ns - ky) % ns;
-  const int a = signed_freq(kx, ns), b = signed_freq(ky, ns);
-  const int na = signed_freq(nkx, ns), nb = signed_freq(nky, ns);
-  float2 h = make_float2(0.f, 0.f);
-  for (int l = 0; l < L; ++l) {
-    const uint64_t ux = up.ux0[l] + (uint64_t)f * up.dux[l];
-    const uint64_t uy = up.uy0[l] + (uint64_t)f * up.duy[l];
-    const float2 x = cmul(spectra[((size_t)l * ns + kx) * ns + ky], phasor2(a, b, ux, uy));
-    const float2 y = cmul(spectra[((size_t)l * ns + nkx) * ns + nky], phasor2(na, nb, ux, uy));
-    h = cadd(h, make_float2(0.5f * (x.x + y.x), 0.5f * (x.y - y.y)));
-  }
-  hn[(size_t)f * 2 * ns + e] = h;
-}
-
-template <int LM, int E>
-__global__ void __launch_bounds__(512)
-k_frame_rows_uniform(FftDesc d, const float2* __restrict__ tw,
-                     const float2* __restrict__ spectra, int L, int F, UniformParams up,
-                     const float2* __restrict__ hn, float2* __restrict__ work) {
-  extern __shared__ float2 sm[];
-  const int ns = d.n;
-  const int kx = blockIdx.x;
-  const int fbeg = blockIdx.y * kAnchor;  // this CTA's frames [fbeg, fbeg + kAnchor)
-  const int vs = fft_buf_len(d) + 1;
-  float2* bufA = sm;
-  float2* bufB = sm + kPairsPerFft * vs;
-  float2* stw = sm + 2 * kPairsPerFft * vs;
-  for (int i = threadIdx.x; i < ns; i += blockDim.x) stw[i] = tw[i];
-  const int kxs = signed_freq(kx, ns), nkx = (ns - kx) % ns;
-  float2 A[E][LM], R[E][LM];
-#pragma unroll
-  for (int e = 0; e < E; ++e) {
-    const int ky = threadIdx.x + e * blockDim.x;
-    const bool live = ky < ns;
-    const int kys = live ? signed_freq(ky, ns) : 0, nky = live ? (ns - ky) % ns : 0;
-#pragma unroll
-    for (int l = 0; l < LM; ++l) {
-      A[e][l] = make_float2(0.f, 0.f);
-      R[e][l] = make_float2(1.f, 0.f);
-      if (l < L && live) {
-        const float2 s = spectra[((size_t)l * ns + kx) * ns + ky];
-        const float2 t = spectra[((size_t)l * ns + nkx) * ns + nky];
-        const float2 sh = make_float2(0.5f * (s.x + t.x), 0.5f * (s.y - t.y));
-        A[e][l] = cmul(sh, phasor2(kxs, kys, up.ux0[l] + (uint64_t)fbeg * up.dux[l],
-                                   up.uy0[l] + (uint64_t)fbeg * up.duy[l]));
-        R[e][l] = phasor2(kxs, kys, up.dux[l], up.duy[l]);
-      }
-    }
-  }
-  const int nfr = min(kAnchor, F - fbeg);
-  const int npairs = (nfr + 1) / 2;
-  for (int pb = 0; pb < npairs; pb += kPairsPerFft) {
-    const int np = min(kPairsPerFft, npairs - pb);
-    for (int p = 0; p < np; ++p) {
-      const bool two = 2 * (pb + p) + 1 < nfr;
-#pragma unroll
-      for (int e = 0; e < E; ++e) {
-        float2 h0a = make_float2(0.f, 0.f), h0b = h0a, h1a = h0a, h1b = h0a;
-#pragma unroll
-        for (int l = 0; l < LM; ++l) {
-          if (l & 1) h0b = cadd(h0b, A[e][l]);
-          else h0a = cadd(h0a, A[e][l]);
-          A[e][l] = cmul(A[e][l], R[e][l]);
-        }
-        if (two) {
-#pragma unroll
-          for (int l = 0; l < LM; ++l) {
-            if (l & 1) h1b = cadd(h1b, A[e][l]);
-            else h1a = cadd(h1a, A[e][l]);
-            A[e][l] = cmul(A[e][l], R[e][l]);
-          }
-        }
-        float2 h0 = cadd(h0a, h0b), h1 = cadd(h1a, h1b);
-        const int ky = threadIdx.x + e * blockDim.x;
-        const bool even = (ns & 1) == 0;
-        if (even && (kx == ns / 2 || ky == ns / 2) && ky < ns) {
-          const int el = kx == ns / 2 ? ky : ns + kx;
-          const int fa = fbeg + 2 * (pb + p);
-          h0 = hn[(size_t)fa * 2 * ns + el];
-          h1 = two ? hn[(size_t)(fa + 1) * 2 * ns + el] : make_float2(0.f, 0.f);
-        }
-        if (ky < ns) bufA[p * vs + ky] = make_float2(h0.x - h1.y, h0.y + h1.x);
-      }
-    }
-    __syncthreads();
-    float2* res = fft_smem(bufA, bufB, d, stw, np, vs, 1, false);
-    for (int i = threadIdx.x; i < np * ns; i += blockDim.x) {
-      const int p = i / ns, c = i % ns;
-      const int pair = fbeg / 2 + pb + p;
-      work[((size_t)pair * ns + kx) * ns + c] = res[p * vs + c];
-    }
-    __syncthreads();
-  }
-}
 
 // ================================================================ pass 2
 // Column transform of a tile of C columns plus the paired real epilogue:
@@ -926,6 +822,91 @@ k_lgs_zoom_tile(int L, int ns, int n, const int32_t* __restrict__ idx, const flo
 #include "gt_fast.cuh"       // register transforms of length 3 * 2^k (Good-Thomas)
 #include "blu_fast.cuh"      // register Bluestein transforms
 
+// Layer sums of equally spaced frames on grids without a fused row kernel:
+// Y[pair][kx][ky] = H_f0 + i H_f1 for every element off the Nyquist cross (the prep
+// launch writes that), to be transformed in place by the row pass of the grid's
+// form. A thread owns a column ky of the row pair {kx, -kx} and advances the
+// recurrence of k_frame_rows_uniform_reg over `run` frames from its exact anchor:
+// half the sums of a kernel that owns one row, and the transforms get the grid's
+// own row pass instead of four rows at a time in shared memory. 64 frames of 9
+// layers on 500^2: 230 us for sums and rows in that kernel, 36 us here and 112 us in
+// the row pass, bound by issue and the stores. Windows of 256 such frames: 500^2
+// 1436 -> 1183 us, 586^2 8703 -> 2357 us, 384^2 925 -> 384 us, 278^2 2015 -> 535 us,
+// 100^2 97 -> 82 us, 128^2 84 -> 54 us, 64^2 62 -> 39 us.
+constexpr int kSumThreads = 128;
+template <int LM>
+__global__ void __launch_bounds__(kSumThreads, LM <= 4 ? 8 : LM <= 9 ? 5 : 4)
+k_uniform_sum(int n, const float2* __restrict__ spectra, int L, int F, int run, UniformTables ut,
+              float2* __restrict__ img) {
+  constexpr int LP = (LM + 1) / 2;  // packed layer pairs
+  const int ky = blockIdx.x * kSumThreads + threadIdx.x, kx = blockIdx.y;
+  const int f0 = blockIdx.z * run, nfr = min(run, F - f0);
+  if (ky >= n || 2 * ky == n) return;
+  const int nkx = kx ? n - kx : 0, nky = ky ? n - ky : 0;
+  f2x Ax[LP], Ay[LP], Rx[LP], Ry[LP], NRy[LP];
+#pragma unroll
+  for (int q = 0; q < LP; ++q) {
+    float ax[2], ay[2], rx[2], ry[2];
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const int l = 2 * q + h;
+      ax[h] = ay[h] = ry[h] = 0.f;
+      rx[h] = 1.f;
+      if (l < LM && l < L) {
+        const float2 sa = spectra[((size_t)l * n + kx) * n + ky];
+        const float2 sb = spectra[((size_t)l * n + nkx) * n + nky];
+        const float2 sh = make_float2(0.5f * (sa.x + sb.x), 0.5f * (sa.y - sb.y));
+        const size_t bl = (size_t)blockIdx.z * L + l;
+        const float2 a = cmul(cmul(sh, ut.px0[bl * n + kx]), ut.py0[bl * n + ky]);
+        const float2 r = cmul(ut.rx[(size_t)l * n + kx], ut.ry[(size_t)l * n + ky]);
+        ax[h] = a.x;
+        ay[h] = a.y;
+        rx[h] = r.x;
+        ry[h] = r.y;
+      }
+    }
+    Ax[q] = pk2(ax[0], ax[1]);
+    Ay[q] = pk2(ay[0], ay[1]);
+    Rx[q] = pk2(rx[0], rx[1]);
+    Ry[q] = pk2(ry[0], ry[1]);
+    NRy[q] = pk2(-ry[0], -ry[1]);
+  }
+  const size_t plane = (size_t)n * n;
+  float2* ra = img + (size_t)(f0 / 2) * plane + (size_t)kx * n + ky;
+  float2* rb = img + (size_t)(f0 / 2) * plane + (size_t)nkx * n + nky;
+  for (int f = 0; f < nfr; f += 2) {
+    float2 h[2];
+#pragma unroll
+    for (int fr = 0; fr < 2; ++fr) {
+      f2x hxa = 0ull, hya = 0ull, hxb = 0ull, hyb = 0ull;
+      if (fr == 0 || f + 1 < nfr) {
+#pragma unroll
+        for (int q = 0; q < LP; ++q) {
+          if (q & 1) {
+            hxb = add2(hxb, Ax[q]);
+            hyb = add2(hyb, Ay[q]);
+          } else {
+            hxa = add2(hxa, Ax[q]);
+            hya = add2(hya, Ay[q]);
+          }
+          const f2x nx = fma2(Ax[q], Rx[q], mul2(Ay[q], NRy[q]));
+          Ay[q] = fma2(Ax[q], Ry[q], mul2(Ay[q], Rx[q]));
+          Ax[q] = nx;
+        }
+      }
+      float a0, a1, b0, b1;
+      upk2(add2(hxa, hxb), a0, a1);
+      upk2(add2(hya, hyb), b0, b1);
+      h[fr] = make_float2(a0 + a1, b0 + b1);
+    }
+    *ra = make_float2(h[0].x - h[1].y, h[0].y + h[1].x);
+    // Y(-k) = conj H0(k) + i conj H1(k)
+    if (kx) *rb = make_float2(h[0].x + h[1].y, h[1].x - h[0].y);
+    ra += plane;
+    rb += plane;
+  }
+}
+
 // Layer sums of frames at arbitrary shifts on grids that are not a power of two:
 // Y[pair][kx][ky] = H_f0 + i H_f1 for every row, to be transformed in place by
 // the row pass of the grid's form. A thread owns one column ky and RB row pairs
@@ -936,7 +917,6 @@ k_lgs_zoom_tile(int L, int ns, int n, const int32_t* __restrict__ idx, const flo
 // of the last block row make the subharmonic coefficients. Five frames of 9
 // layers on 728^2 took 81.6 us for coefficients, phasor tables and rows in one
 // shared-memory kernel, 44.3 us in this one and the row pass.
-constexpr int kSumThreads = 128;
 template <int NF, int RB, int CAP>
 __global__ void __launch_bounds__(kSumThreads)
 k_frame_sum(int n, const float2* __restrict__ spectra, const __grid_constant__ FramePrepArgs a,
@@ -1038,16 +1018,14 @@ static size_t cols_smem(int ns, int nb, int C, int P) {
 }
 
 // The grid's transform for the frame passes: the Bluestein form only when
-// its buffers fit (the frame row kernels hold eight and 2 x kPairsPerFft
-// rows); otherwise the direct-sum stages.
+// its buffers fit (the frame row kernel holds eight rows); otherwise the
+// direct-sum stages.
 static FftDesc frame_desc(const pt_grid* g) {
   FftDesc d = g->desc;
   const int ns = g->ns;
   if (d.M > 0) {
     const size_t cap = 220 * 1024;
-    if (frame_rows_smem(ns, d.M) > cap ||
-        (size_t)(2 * kPairsPerFft * (d.M + 1) + ns) * sizeof(float2) > cap ||
-        cols_smem(ns, d.M, cols_per_cta(d.M), g->P) > cap)
+    if (frame_rows_smem(ns, d.M) > cap || cols_smem(ns, d.M, cols_per_cta(d.M), g->P) > cap)
       d.M = 0;
   }
   return d;
@@ -1102,56 +1080,6 @@ static bool uniform_ok(const double* sx, const double* sy, int per_layer, int L,
   return true;
 }
 
-template <int LM>
-static int launch_uniform_t(const pt_grid* g, const float2* spectra, int L, int nf,
-                            const UniformParams& up, float2* hn, float2* ptab, float2* img,
-                            cudaStream_t s) {
-  const int ns = g->ns;
-  if ((ns & 1) == 0) {
-    k_nyquist_h<<<dim3((2 * ns + 127) / 128, nf), 128, 0, s>>>(ns, spectra, L, nf, up, hn);
-    count_launch();
-  }
-  const dim3 grid(ns, (nf + kAnchor - 1) / kAnchor);
-  ProfScope ps("k_frame_rows_uniform", s);
-  (void)ptab;  // the power-of-two sizes 256/512/1024 take launch_uniform_reg_chunk instead
-  const FftDesc fd = frame_desc(g);
-  const size_t smem = (size_t)(2 * kPairsPerFft * (fft_buf_len(fd) + 1) + ns) * sizeof(float2);
-  if (ns <= 512) {
-    if (int rc = set_smem(k_frame_rows_uniform<LM, 1>, smem, "k_frame_rows_uniform")) return rc;
-    k_frame_rows_uniform<LM, 1><<<grid, ns, smem, s>>>(fd, g->tw, spectra, L, nf, up, hn,
-                                                       img);
-  } else {
-    if (int rc = set_smem(k_frame_rows_uniform<LM, 2>, smem, "k_frame_rows_uniform")) return rc;
-    k_frame_rows_uniform<LM, 2><<<grid, (ns + 1) / 2, smem, s>>>(fd, g->tw, spectra, L, nf,
-                                                                up, hn, img);
-  }
-  return PT_OK;
-}
-
-static int launch_uniform_rows(const pt_grid* g, const float2* spectra, int L, const double* sx,
-                               const double* sy, int f0, int nf, float2* hn, float2* ptab,
-                               float2* img, cudaStream_t s) {
-  const double df = 1.0 / (g->ns * g->dx);
-  UniformParams up{};
-  for (int l = 0; l < L; ++l) {
-    const double x0 = sx[(size_t)f0 * L + l], y0 = sy[(size_t)f0 * L + l];
-    const double dx = (sx[(size_t)(f0 + nf - 1) * L + l] - x0) / (nf - 1);
-    const double dy = (sy[(size_t)(f0 + nf - 1) * L + l] - y0) / (nf - 1);
-    up.ux0[l] = host_fixed(x0 * df);
-    up.uy0[l] = host_fixed(y0 * df);
-    up.dux[l] = host_fixed(dx * df);
-    up.duy[l] = host_fixed(dy * df);
-  }
-  if (L <= 1) return launch_uniform_t<1>(g, spectra, L, nf, up, hn, ptab, img, s);
-  if (L <= 2) return launch_uniform_t<2>(g, spectra, L, nf, up, hn, ptab, img, s);
-  if (L <= 3) return launch_uniform_t<3>(g, spectra, L, nf, up, hn, ptab, img, s);
-  if (L <= 4) return launch_uniform_t<4>(g, spectra, L, nf, up, hn, ptab, img, s);
-  if (L <= 6) return launch_uniform_t<6>(g, spectra, L, nf, up, hn, ptab, img, s);
-  if (L <= 9) return launch_uniform_t<9>(g, spectra, L, nf, up, hn, ptab, img, s);
-  if (L <= 12) return launch_uniform_t<12>(g, spectra, L, nf, up, hn, ptab, img, s);
-  return launch_uniform_t<16>(g, spectra, L, nf, up, hn, ptab, img, s);
-}
-
 // ---- uniform frames on the 256/512/1024 register path: one prep launch + rows
 template <int LM>
 static int uniform_reg_rows_t(const pt_grid* g, const float2* spectra, int L, int nf,
@@ -1171,9 +1099,11 @@ static int uniform_reg_rows_t(const pt_grid* g, const float2* spectra, int L, in
   return go(k_frame_rows_uniform_reg<LM, 1024>, 512, 4);
 }
 
-static int launch_uniform_reg_chunk(const pt_grid* g, const float2* spectra, const float2* sh_coef,
-                                    int L, const double* sx, const double* sy, int f0, int nf,
-                                    const SpecWork& w, cudaStream_t s) {
+// tables, Nyquist cross and subharmonic coefficients of frames [f0, f0 + nf), an
+// anchor every `run` frames; the cross goes to w.hn, or with `direct` to the images
+static int launch_uniform_prep(const pt_grid* g, const float2* spectra, const float2* sh_coef,
+                               int L, const double* sx, const double* sy, int f0, int nf, int run,
+                               bool direct, const SpecWork& w, UniformTables* ut, cudaStream_t s) {
   const int ns = g->ns;
   const double df = 1.0 / (ns * g->dx);
   UniformPrep a{};
@@ -1190,7 +1120,7 @@ static int launch_uniform_reg_chunk(const pt_grid* g, const float2* spectra, con
     a.dsx[l] = dx;
     a.dsy[l] = dy;
   }
-  const int nb = (nf + kAnchor - 1) / kAnchor;
+  const int nb = (nf + run - 1) / run;
   float2* ptab = w.px;
   a.px0 = ptab;
   a.py0 = ptab + (size_t)nb * L * ns;
@@ -1208,14 +1138,25 @@ static int launch_uniform_reg_chunk(const pt_grid* g, const float2* spectra, con
   a.P = g->P;
   a.F = nf;
   a.nb = nb;
+  a.run = run;
+  a.img = direct ? w.img : nullptr;
   a.blocks_tab = ((nb + 1) * L * ns + 255) / 256;
-  a.blocks_nyq = (2 * ns * ((nf + kNyqGroup - 1) / kNyqGroup) + 255) / 256;
+  a.blocks_nyq = ns & 1 ? 0 : (2 * ns * ((nf + kNyqGroup - 1) / kNyqGroup) + 255) / 256;
   {
     ProfScope ps("k_uniform_prep", s);
     k_uniform_prep<<<a.blocks_tab + a.blocks_nyq + nf, 256, 0, s>>>(a);
   }
   count_launch();
-  const UniformTables ut{a.px0, a.py0, a.rx, a.ry};
+  *ut = UniformTables{a.px0, a.py0, a.rx, a.ry};
+  return PT_OK;
+}
+
+static int launch_uniform_reg_chunk(const pt_grid* g, const float2* spectra, const float2* sh_coef,
+                                    int L, const double* sx, const double* sy, int f0, int nf,
+                                    const SpecWork& w, cudaStream_t s) {
+  UniformTables ut;
+  if (int rc = launch_uniform_prep(g, spectra, sh_coef, L, sx, sy, f0, nf, kAnchor, false, w, &ut, s))
+    return rc;
   if (L <= 1) return uniform_reg_rows_t<1>(g, spectra, L, nf, ut, w.hn, w.img, s);
   if (L <= 2) return uniform_reg_rows_t<2>(g, spectra, L, nf, ut, w.hn, w.img, s);
   if (L <= 3) return uniform_reg_rows_t<3>(g, spectra, L, nf, ut, w.hn, w.img, s);
@@ -1224,6 +1165,35 @@ static int launch_uniform_reg_chunk(const pt_grid* g, const float2* spectra, con
   if (L <= 9) return uniform_reg_rows_t<9>(g, spectra, L, nf, ut, w.hn, w.img, s);
   if (L <= 12) return uniform_reg_rows_t<12>(g, spectra, L, nf, ut, w.hn, w.img, s);
   return uniform_reg_rows_t<16>(g, spectra, L, nf, ut, w.hn, w.img, s);
+}
+
+// ---- uniform frames on other grids: layer sums, to be transformed by the row pass
+template <int LM>
+static int uniform_sum_t(const pt_grid* g, const float2* spectra, int L, int nf, int run,
+                         const UniformTables& ut, float2* img, cudaStream_t s) {
+  const int n = g->ns;
+  ProfScope ps("k_uniform_sum", s);
+  k_uniform_sum<LM><<<dim3((n + kSumThreads - 1) / kSumThreads, (n + 1) / 2, (nf + run - 1) / run),
+                      kSumThreads, 0, s>>>(n, spectra, L, nf, run, ut, img);
+  count_launch();
+  return PT_OK;
+}
+static int launch_uniform_sum(const pt_grid* g, const float2* spectra, const float2* sh_coef, int L,
+                              const double* sx, const double* sy, int f0, int nf, const SpecWork& w,
+                              cudaStream_t s) {
+  // frames in runs, each from its own anchor: as few as give every SM ten CTAs,
+  // but of eight frames at least (the spectra are read once a run)
+  const int n = g->ns, ctas = (n + kSumThreads - 1) / kSumThreads * ((n + 1) / 2);
+  const int runs = std::min(8, (1520 + ctas - 1) / ctas);
+  const int run = std::max(8, ((nf + runs - 1) / runs + 1) & ~1);
+  UniformTables ut;
+  if (int rc = launch_uniform_prep(g, spectra, sh_coef, L, sx, sy, f0, nf, run, true, w, &ut, s)) return rc;
+  if (L <= 2) return uniform_sum_t<2>(g, spectra, L, nf, run, ut, w.img, s);
+  if (L <= 4) return uniform_sum_t<4>(g, spectra, L, nf, run, ut, w.img, s);
+  if (L <= 6) return uniform_sum_t<6>(g, spectra, L, nf, run, ut, w.img, s);
+  if (L <= 9) return uniform_sum_t<9>(g, spectra, L, nf, run, ut, w.img, s);
+  if (L <= 12) return uniform_sum_t<12>(g, spectra, L, nf, run, ut, w.img, s);
+  return uniform_sum_t<16>(g, spectra, L, nf, run, ut, w.img, s);
 }
 
 // shifts of global frames [f0, f0 + nf), term by term
@@ -2078,8 +2048,16 @@ extern "C" int pt_frames(const pt_grid* g, int L, const float* spectra, const fl
     if (sum) {
       // phasors, layer sums and coefficients, then the grid's own row pass in place
       if (int rc = launch_frame_sum(g, (const float2*)spectra, pa, sx, sy, f0, w.img, s)) return rc;
+    } else if (uni && !uni_reg) {
+      if (int rc = launch_uniform_sum(g, (const float2*)spectra, (const float2*)sh_coef, L, sx, sy, f0,
+                                      nf, w, s))
+        return rc;
+    }
+    if (sum || (uni && !uni_reg)) {
       const GenRowArgs none{};
-      if (blu) {
+      if (pow2_fast(ns)) {
+        if (int rc = rows_reg(g, w.img, 0, none, npair, w.img, s)) return rc;
+      } else if (blu) {
         if (int rc = rows_blu(g->desc, w.img, 0, none, npair, w.img, s)) return rc;
       } else if (gt_m(ns)) {
         if (int rc = rows_gt(g, w.img, 0, none, npair, w.img, s)) return rc;
@@ -2092,7 +2070,7 @@ extern "C" int pt_frames(const pt_grid* g, int L, const float* spectra, const fl
                                                                        none, w.img);
       }
     }
-    for (int fb = 0; fb < nf && !uni_reg && !reg && !sum; fb += fsub) {
+    for (int fb = 0; fb < nf && !uni && !reg && !sum; fb += fsub) {
       const int nb = std::min(fsub, nf - fb);
       ShiftParams sp;
       for (int f = 0; f < nb; ++f)
@@ -2106,18 +2084,11 @@ extern "C" int pt_frames(const pt_grid* g, int L, const float* spectra, const fl
         k_frame_coef<<<nb, 32 * ((P * 9 + 31) / 32), 0, s>>>(pa, sp, fb, nb);
         count_launch();
       }
-      if (uni) continue;  // no phasor tables needed
       ProfScope ps("k_frame_phasors", s);
       k_frame_phasors<<<dim3((ns + 255) / 256, nb * J), 256, 0, s>>>(pa, sp, fb);
       count_launch();
     }
-    if (uni_reg || reg || sum) {
-      // rows done above
-    } else if (uni) {
-      if (int rc = launch_uniform_rows(g, (const float2*)spectra, L, sx, sy, f0, nf, w.hn, w.px,
-                                       w.img, s))
-        return rc;
-    } else {
+    if (!uni && !reg && !sum) {
       FrameRowArgs fa{(const float2*)spectra, w.px, w.py, J, nf, f0, per_layer};
       if (int rc = set_smem(k_frame_rows, rs, "k_frame_rows")) return rc;
       ProfScope ps("k_frame_rows", s);
