@@ -295,7 +295,18 @@ static __device__ __noinline__ void stage_prime(const float2* a, float2* b, cons
   else stage_r<13>(a, b, tw, n, Ns, nvec, vs, es, vfast);
 }
 
-// The Stockham stages of a length-n transform with the given radices.
+// Whether a plan has a stage of radix 7, 11 or 13.
+inline bool fft_primes(const FftDesc& d) {
+  for (int s = 0; s < d.nstages; ++s)
+    if (d.radix[s] == 7 || d.radix[s] == 11 || d.radix[s] == 13) return true;
+  return false;
+}
+
+// The Stockham stages of a length-n transform with the given radices. Kernels for
+// plans without the primes above leave those stages out: they cost 16 to 24 registers
+// a thread even where no stage runs them (100 screens of 144^2: 52 us with, 42 us
+// without; 20 of 600^2: 144 and 140 us; 30 of 300^2: 69 and 55 us).
+template <bool PRIME = true>
 __device__ inline float2* fft_stages(float2* a, float2* b, const int* radix, int nstages,
                                      const float2* tw, int n, int nvec, int vs, int es,
                                      bool vfast) {
@@ -307,11 +318,11 @@ __device__ inline float2* fft_stages(float2* a, float2* b, const int* radix, int
       case 3: stage_r<3>(a, b, tw, n, Ns, nvec, vs, es, vfast); break;
       case 4: stage_r<4>(a, b, tw, n, Ns, nvec, vs, es, vfast); break;
       case 5: stage_r<5>(a, b, tw, n, Ns, nvec, vs, es, vfast); break;
-      case 7: stage_r<7>(a, b, tw, n, Ns, nvec, vs, es, vfast); break;
       case 8: stage_r<8>(a, b, tw, n, Ns, nvec, vs, es, vfast); break;
-      case 11:
-      case 13: stage_prime(a, b, tw, n, R, Ns, nvec, vs, es, vfast); break;
-      default: stage_generic(a, b, tw, n, R, Ns, nvec, vs, es); break;
+      default:
+        if (PRIME && R == 7) stage_r<7>(a, b, tw, n, Ns, nvec, vs, es, vfast);
+        else if (PRIME && (R == 11 || R == 13)) stage_prime(a, b, tw, n, R, Ns, nvec, vs, es, vfast);
+        else stage_generic(a, b, tw, n, R, Ns, nvec, vs, es);
     }
     __syncthreads();
     float2* t = a;
@@ -336,7 +347,7 @@ __device__ inline float2* fft_bluestein(float2* a, float2* b, const FftDesc& d, 
     *p = e < n ? cmul(*p, __ldg(d.chirp + e)) : make_float2(0.f, 0.f);
   }
   __syncthreads();
-  float2* x = fft_stages(a, b, d.mradix, d.mstages, d.twM, M, nvec, vs, es, vfast);
+  float2* x = fft_stages<false>(a, b, d.mradix, d.mstages, d.twM, M, nvec, vs, es, vfast);
   float2* y = x == a ? b : a;
   for (int t = threadIdx.x; t < nvec * M; t += blockDim.x) {
     const int v = vfast ? t % nvec : t / M, e = vfast ? t / nvec : t % M;
@@ -344,7 +355,7 @@ __device__ inline float2* fft_bluestein(float2* a, float2* b, const FftDesc& d, 
     *p = cconj(cmul(*p, __ldg(d.bhat + e)));
   }
   __syncthreads();
-  float2* z = fft_stages(x, y, d.mradix, d.mstages, d.twM, M, nvec, vs, es, vfast);
+  float2* z = fft_stages<false>(x, y, d.mradix, d.mstages, d.twM, M, nvec, vs, es, vfast);
   const float inv = 1.0f / (float)M;
   for (int t = threadIdx.x; t < nvec * n; t += blockDim.x) {
     const int v = vfast ? t % nvec : t / n, e = vfast ? t / nvec : t % n;
@@ -359,10 +370,11 @@ __device__ inline float2* fft_bluestein(float2* a, float2* b, const FftDesc& d, 
 // v sits at buf[v * vs + e * es]; both buffers hold fft_buf_len(d) elements
 // a vector. Returns the buffer holding the result (a or b). Ends with
 // __syncthreads().
+template <bool PRIME = true>
 __device__ inline float2* fft_smem(float2* a, float2* b, const FftDesc& d, const float2* tw,
                                    int nvec, int vs, int es, bool vfast) {
   if (d.M > 0) return fft_bluestein(a, b, d, nvec, vs, es, vfast);
-  return fft_stages(a, b, d.radix, d.nstages, tw, d.n, nvec, vs, es, vfast);
+  return fft_stages<PRIME>(a, b, d.radix, d.nstages, tw, d.n, nvec, vs, es, vfast);
 }
 
 }  // namespace pt

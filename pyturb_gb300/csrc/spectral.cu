@@ -70,10 +70,19 @@ static inline int gen_chunk(int ns) {
   return (int)std::max<size_t>(1, std::min<size_t>(256, c));
 }
 // Rows / columns a CTA of the shared-memory passes transforms, from the buffer
-// length (fft_buf_len: M for a Bluestein grid): about 4096 elements a CTA, so that
-// the stages of the larger radices still give most threads a butterfly. Rows of
-// three 728^2 images: 25.4 us at 2048 elements, 20.4 us so.
-static inline int rows_per_cta(int nb) { return std::max(1, std::min(16, 4096 / nb)); }
+// length (fft_buf_len: M for a Bluestein grid): about 4096 elements of columns, and
+// of rows 3072 (more CTAs to fill the last wave; 4096 in brackets: 8 screens of
+// 700^2 81 (83) us, 4 of 1000^2 91 (95) us, three images of 728^2 2 us more) or, of
+// vectors below 320 elements, 2048 (3072 in brackets: 100 screens of 200^2 71 (73)
+// us, 20 of 250^2 42 (44) us, but 64 of 280^2 89 (85) us). A frame pass over `nimg`
+// images takes the 4096 where that makes its rows one wave of three CTAs an SM (five
+// directions on 728^2: 95 us without, 90 us so).
+static inline int rows_per_cta(int nb, int ns = 0, int nimg = 0) {
+  const int r = std::max(1, std::min(16, (nb < 320 ? 2048 : 3072) / nb));
+  const int r2 = std::max(1, std::min(16, 4096 / nb));
+  const auto ctas = [&](int q) { return (long long)((ns + q - 1) / q) * nimg; };
+  return ctas(r) > 3 * 152 && ctas(r2) <= 3 * 152 ? r2 : r;
+}
 static inline int cols_per_cta(int nb) { return std::max(1, std::min(16, 4096 / nb)); }
 // The shape of a column pass over `nimg` images: where such CTAs would not fill
 // the SMs three times over, more columns and threads a CTA (three 728^2 images:
@@ -190,6 +199,7 @@ __device__ __forceinline__ void gen_coef_pair(const GenRowArgs& a, int img) {
 // Plain complex rows (pt_ifft2; frames, in place) and generate rows share this
 // kernel: `gen` selects the producer. rpc rows per CTA, one transform per row; a
 // CTA has read its rows before it writes them, so `in` may be `work`.
+template <bool PRIME>
 __global__ void __launch_bounds__(kThreads)
 k_rows(FftDesc d, const float2* __restrict__ tw, int rpc, const float2* in,
        int gen, GenRowArgs ga, float2* work) {
@@ -226,7 +236,7 @@ k_rows(FftDesc d, const float2* __restrict__ tw, int rpc, const float2* in,
     bufA[r * vs + ky] = v;
   }
   __syncthreads();
-  float2* res = fft_smem(bufA, bufB, d, stw, rpc, vs, 1, false);
+  float2* res = fft_smem<PRIME>(bufA, bufB, d, stw, rpc, vs, 1, false);
   for (int i = threadIdx.x; i < rpc * ns; i += blockDim.x) {
     const int r = i / ns, ky = i % ns;
     const int kx = row0 + r;
@@ -356,7 +366,7 @@ __device__ __forceinline__ float img_scale_of(const PairStore& st, int img) {
   return st.img_scale ? st.scale * __ldg(st.img_scale + img) : st.scale;
 }
 
-template <int THREADS>
+template <int THREADS, bool PRIME>
 __global__ void __launch_bounds__(THREADS)
 k_pair_cols(FftDesc d, const float2* __restrict__ tw, const float2* __restrict__ work, int C,
             int pair0, PairStore st) {
@@ -429,7 +439,7 @@ k_pair_cols(FftDesc d, const float2* __restrict__ tw, const float2* __restrict__
       for (int i = threadIdx.x; i < P * ns; i += blockDim.x)
         sbasis[i] = __ldg(st.basis + (size_t)(3 * (i / ns)) * ns + (i % ns));
   }
-  float2* res = fft_smem(bufA, bufB, d, stw, C, 1, C, true);
+  float2* res = fft_smem<PRIME>(bufA, bufB, d, stw, C, 1, C, true);
   const float mre = (P > 0 && do_re) ? st.mean[row_re] : 0.f;
   const float mim = (P > 0 && do_im) ? st.mean[row_im] : 0.f;
   const float sre = img_scale_of(st, img_re), sim = img_scale_of(st, img_im);
@@ -472,6 +482,14 @@ k_pair_cols(FftDesc d, const float2* __restrict__ tw, const float2* __restrict__
       if (do_im) __stcs(st.out + (size_t)img_im * plane + o, sim * (v.y + lim));
     }
   }
+}
+
+using RowsKernel = void (*)(FftDesc, const float2*, int, const float2*, int, GenRowArgs, float2*);
+static RowsKernel rows_kernel(const FftDesc& d) { return fft_primes(d) ? k_rows<true> : k_rows<false>; }
+using PairColsKernel = void (*)(FftDesc, const float2*, const float2*, int, int, PairStore);
+template <int THREADS>
+static PairColsKernel pair_cols_kernel(const FftDesc& d) {
+  return fft_primes(d) ? k_pair_cols<THREADS, true> : k_pair_cols<THREADS, false>;
 }
 
 // plain complex column pass (pt_ifft2)
@@ -1838,7 +1856,7 @@ extern "C" int pt_ifft2(const pt_grid* g, const float* in, float* out, int batch
   const size_t rs = rows_smem(ns, blen, rpc), cs = cols_smem(ns, blen, C, 0);
   const bool blu = blu_fast(g->desc);
   if (!pow2_fast(ns) && !blu) {
-    if (int rc = set_smem(k_rows, rs, "k_rows")) return rc;
+    if (int rc = set_smem(rows_kernel(g->desc), rs, "k_rows")) return rc;
     if (int rc = set_smem(k_plain_cols, cs, "k_plain_cols")) return rc;
   }
   GenRowArgs none{};
@@ -1855,7 +1873,7 @@ extern "C" int pt_ifft2(const pt_grid* g, const float* in, float* out, int batch
     } else {
       {
         ProfScope ps("k_rows", s);
-        k_rows<<<dim3((ns + rpc - 1) / rpc, nb), kThreads, rs, s>>>(g->desc, g->tw, rpc, src, 0,
+        rows_kernel(g->desc)<<<dim3((ns + rpc - 1) / rpc, nb), kThreads, rs, s>>>(g->desc, g->tw, rpc, src, 0,
                                                                    none, w.img);
       }
       ProfScope ps("k_plain_cols", s);
@@ -1888,8 +1906,8 @@ static int generate_impl(const pt_grid* g, int count, const float* amplitude,
   const size_t rs = rows_smem(ns, blen, rpc), cs = cols_smem(ns, blen, C, P);
   const bool blu = blu_fast(g->desc);
   if (!pow2_fast(ns) && !gt_m(ns) && !blu) {
-    if (int rc = set_smem(k_rows, rs, "k_rows")) return rc;
-    if (int rc = set_smem(k_pair_cols<kThreads>, cs, "k_pair_cols")) return rc;
+    if (int rc = set_smem(rows_kernel(g->desc), rs, "k_rows")) return rc;
+    if (int rc = set_smem(pair_cols_kernel<kThreads>(g->desc), cs, "k_pair_cols")) return rc;
   }
   for (int b0 = 0; b0 < n_fft; b0 += ch) {
     const int nb = std::min(ch, n_fft - b0);
@@ -1903,7 +1921,7 @@ static int generate_impl(const pt_grid* g, int count, const float* amplitude,
       if (int rc = rows_blu(g->desc, nullptr, 1, ga, nb, w.img, s)) return rc;
     } else {
       ProfScope ps("k_rows", s);
-      k_rows<<<dim3((ns + rpc - 1) / rpc, nb), kThreads, rs, s>>>(g->desc, g->tw, rpc, nullptr, 1,
+      rows_kernel(g->desc)<<<dim3((ns + rpc - 1) / rpc, nb), kThreads, rs, s>>>(g->desc, g->tw, rpc, nullptr, 1,
                                                                  ga, w.img);
     }
     count_launch();
@@ -1935,7 +1953,7 @@ static int generate_impl(const pt_grid* g, int count, const float* amplitude,
       if (int rc = cols_blu(g, g->desc, w.img, nb, b0, &st, nullptr, s)) return rc;
     } else {
       ProfScope ps("k_pair_cols", s);
-      k_pair_cols<kThreads><<<dim3((ns + C - 1) / C, nb), kThreads, cs, s>>>(g->desc, g->tw, w.img, C, b0, st);
+      pair_cols_kernel<kThreads>(g->desc)<<<dim3((ns + C - 1) / C, nb), kThreads, cs, s>>>(g->desc, g->tw, w.img, C, b0, st);
     }
     count_launch();
     if (int rc = check_launch("pt_generate")) return rc;
@@ -2062,11 +2080,11 @@ extern "C" int pt_frames(const pt_grid* g, int L, const float* spectra, const fl
       } else if (gt_m(ns)) {
         if (int rc = rows_gt(g, w.img, 0, none, npair, w.img, s)) return rc;
       } else {
-        const int rb = fft_buf_len(g->desc), rpc = rows_per_cta(rb);
+        const int rb = fft_buf_len(g->desc), rpc = rows_per_cta(rb, ns, npair);
         const size_t rsm = rows_smem(ns, rb, rpc);
-        if (int rc = set_smem(k_rows, rsm, "k_rows")) return rc;
+        if (int rc = set_smem(rows_kernel(g->desc), rsm, "k_rows")) return rc;
         ProfScope ps("k_rows", s);
-        k_rows<<<dim3((ns + rpc - 1) / rpc, npair), kThreads, rsm, s>>>(g->desc, g->tw, rpc, w.img, 0,
+        rows_kernel(g->desc)<<<dim3((ns + rpc - 1) / rpc, npair), kThreads, rsm, s>>>(g->desc, g->tw, rpc, w.img, 0,
                                                                        none, w.img);
       }
     }
@@ -2126,11 +2144,11 @@ extern "C" int pt_frames(const pt_grid* g, int L, const float* spectra, const fl
       const size_t csm = cols_smem(ns, blen, sh.C, P);
       const dim3 grid((ns + sh.C - 1) / sh.C, npair);
       if (sh.threads == kThreads) {
-        if (int rc = set_smem(k_pair_cols<kThreads>, csm, "k_pair_cols")) return rc;
-        k_pair_cols<kThreads><<<grid, kThreads, csm, s>>>(fd, g->tw, w.img, sh.C, 0, st);
+        if (int rc = set_smem(pair_cols_kernel<kThreads>(fd), csm, "k_pair_cols")) return rc;
+        pair_cols_kernel<kThreads>(fd)<<<grid, kThreads, csm, s>>>(fd, g->tw, w.img, sh.C, 0, st);
       } else {
-        if (int rc = set_smem(k_pair_cols<kColThreads>, csm, "k_pair_cols")) return rc;
-        k_pair_cols<kColThreads><<<grid, kColThreads, csm, s>>>(fd, g->tw, w.img, sh.C, 0, st);
+        if (int rc = set_smem(pair_cols_kernel<kColThreads>(fd), csm, "k_pair_cols")) return rc;
+        pair_cols_kernel<kColThreads>(fd)<<<grid, kColThreads, csm, s>>>(fd, g->tw, w.img, sh.C, 0, st);
       }
     }
     count_launch();
@@ -2273,7 +2291,7 @@ extern "C" int pt_ifft2_noalloc(int ns, const float* in, float* out, int batch, 
   const int rpc = rows_per_cta(ns), C = cols_per_cta(ns);  // no Bluestein form here
   const size_t rs = rows_smem(ns, ns, rpc), cs = cols_smem(ns, ns, C, 0);
   if (!pow2_fast(ns)) {
-    if (int rc = set_smem(k_rows, rs, "k_rows")) return rc;
+    if (int rc = set_smem(rows_kernel(g.desc), rs, "k_rows")) return rc;
     if (int rc = set_smem(k_plain_cols, cs, "k_plain_cols")) return rc;
   }
   GenRowArgs none{};
@@ -2285,7 +2303,7 @@ extern "C" int pt_ifft2_noalloc(int ns, const float* in, float* out, int batch, 
       if (int rc = rows_reg(&g, src, 0, none, nb, scratch, s)) return rc;
       if (int rc = plain_cols_reg(&g, scratch, nb, dst, s)) return rc;
     } else {
-      k_rows<<<dim3((ns + rpc - 1) / rpc, nb), kThreads, rs, s>>>(g.desc, g.tw, rpc, src, 0, none,
+      rows_kernel(g.desc)<<<dim3((ns + rpc - 1) / rpc, nb), kThreads, rs, s>>>(g.desc, g.tw, rpc, src, 0, none,
                                                                  scratch);
       k_plain_cols<<<dim3((ns + C - 1) / C, nb), kThreads, cs, s>>>(g.desc, g.tw, scratch, C, dst);
     }
