@@ -952,7 +952,7 @@ def main() -> None:
                      "frac": gbs / hbm, "bytes_per_screen": n_px * n_px * 4,
                      "workload": f"{n_px}^2 screens, {prof_note}",
                      "note": "issue-bound kernels (Philox + Box-Muller + register FFT rows; "
-                             "barrier-bound 1024-thread column pass): profiles/"
+                             "column pass pipelined over tiles): profiles/"
                              "generate_512_mc.md"}
     line["dft_512_tc_vs_fp32"] = bench_tc_dft(torch)
     if not args.no_extrude:
