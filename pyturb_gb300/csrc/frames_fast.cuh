@@ -66,11 +66,11 @@ __device__ __forceinline__ f2x add2(f2x a, f2x b) {
 }
 
 // ------------------------------------------------------------------ rows
-// plain complex input (pt_ifft2) or generate's coloured noise
+// plain complex input (pt_ifft2; frames, in place: a team reads its row before it
+// writes it, so `in` may be `work`) or generate's coloured noise
 template <int N>
 __global__ void __launch_bounds__(RegCfg<N>::THREADS)
-k_rows_reg(const float2* __restrict__ tw, const float2* __restrict__ in, int gen, GenRowArgs ga,
-           float2* __restrict__ work) {
+k_rows_reg(const float2* __restrict__ tw, const float2* in, int gen, GenRowArgs ga, float2* work) {
   constexpr int T = RegCfg<N>::T, NV = RegCfg<N>::NV;
   extern __shared__ float2 sm[];
   float2* stw = sm;
