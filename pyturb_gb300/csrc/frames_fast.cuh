@@ -434,7 +434,7 @@ k_pair_cols_pipe(const float2* __restrict__ tw, const float2* work, int npair, i
         x[i].y = fmaf(b.x, u.z, fmaf(b.y, u.w, x[i].y));
       }
     }
-    const float sre = do_re ? img_scale_of(st, img_re) : 0.f, sim = do_im ? img_scale_of(st, img_im) : 0.f;
+    const float sre = img_scale_of(st, img_re), sim = img_scale_of(st, img_im);
     float* ore = st.out + (size_t)(do_re ? img_re : 0) * plane + yo;
     float* oim = st.out + (size_t)(do_im ? img_im : 0) * plane + yo;
 #pragma unroll

@@ -362,8 +362,9 @@ struct PairStore {
   const float* img_scale;  // per output image factor on top of `scale` (NULL: none)
 };
 
+// (An odd count's last pair has one image: the table ends before the other.)
 __device__ __forceinline__ float img_scale_of(const PairStore& st, int img) {
-  return st.img_scale ? st.scale * __ldg(st.img_scale + img) : st.scale;
+  return st.img_scale && img < st.count ? st.scale * __ldg(st.img_scale + img) : st.scale;
 }
 
 template <int THREADS, bool PRIME>
