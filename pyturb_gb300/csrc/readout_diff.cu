@@ -35,6 +35,7 @@ static inline void count_launch_r(int k = 1) {
 constexpr int kLrMaxLayers = 32;
 constexpr int kLrMaxMag = 256;   // D * L entries of the magnification table
 constexpr int kLrBand = 64;      // pupil rows per CTA (forward, parameter gradients)
+constexpr int kLrTogether = 10;  // layers of a forward launch
 constexpr long long kLrOne = 1ll << 32;
 
 struct LrMag {
@@ -92,9 +93,9 @@ __device__ __forceinline__ float ld_at(const float* base, uint32_t byte_off) {
 }
 
 // Row tables of NL layers l0, l0 + 1, ... (clamped to L - 1) for a band of
-// pupil rows: byte offsets of the upper and lower sample row inside the
-// (L, S, S) screens of one realisation, and the fraction between them. Layers
-// are adjacent, so a thread reads a row's entries with 16-byte loads.
+// pupil rows: byte offsets of the upper and lower sample row from a realisation's
+// first screen of the launch, and the fraction between them. Layers are adjacent, so
+// a thread reads a row's entries with 16-byte loads.
 template <int NL>
 struct BandTab {
   static constexpr int NP = (NL + 3) & ~3;
@@ -135,9 +136,13 @@ __device__ __forceinline__ bool all_unit(const long long* __restrict__ fx, int l
 }
 
 // Forward: CTA = (band of kLrBand pupil rows, t*D + d, b); threads walk
-// columns, then the rows of the band, the NL = L layers of a pixel together
-// (k_lr_forward_any takes more layers than the instantiated ones, and screens
-// whose byte offsets pass 32 bits).
+// columns, then the rows of the band, the NL layers of a pixel together. A launch
+// takes at most kLrTogether of the L layers and as many as 32-bit byte offsets reach;
+// screens, w and fix start at its first layer. A further launch (ADD) adds its layers
+// to the output, which keeps the order of the sum: 16 layers in 8 + 8 took 76 us for
+// 2 x 2 frames of 4 directions, 768^2 screens, 512^2 pupils, and 452 us in one form
+// for up to 32 layers. (k_lr_forward_any takes the screens that pass 32 bits by
+// themselves.)
 //
 // Bound by instruction issue and the L1 data path (scattered 4-byte taps; issue
 // active 75%, L1 68%). Where every layer of the image has unit magnification
@@ -148,20 +153,20 @@ __device__ __forceinline__ bool all_unit(const long long* __restrict__ fx, int l
 // 32-bit offsets take the address and predicate instructions from 45 a sample
 // to 16. 4 x 8 frames of 9 directions, 9 layers, 768^2 screens, 512^2 pupils:
 // 1093 us with four loads and 64-bit offsets, 411 us so.
-template <int NL>
+template <int NL, bool ADD>
 __global__ void __launch_bounds__(256, NL <= 6 ? 3 : 2)
-k_lr_forward(int S, int T, int D, int n, const float* __restrict__ screens,
+k_lr_forward(int L, int S, int T, int D, int n, const float* __restrict__ screens,
              const float* __restrict__ w, const long long* __restrict__ fix,
              float* __restrict__ out) {
   __shared__ BandTab<NL> tab;
   const int band0 = blockIdx.x * kLrBand;
   const int td = blockIdx.y, b = blockIdx.z;
   const int rows = min(kLrBand, n - band0);
-  const long long* fx = fix + (size_t)td * NL * 3;
+  const long long* fx = fix + (size_t)td * L * 3;
   const bool unit = all_unit<NL>(fx, 0, NL);
   band_table<NL>(tab, fx, 0, NL, S, band0);
   __syncthreads();
-  const float* scr = screens + (size_t)b * NL * S * S;
+  const float* scr = screens + (size_t)b * L * S * S;
   float* o = out + ((size_t)b * T * D + td) * n * n + (size_t)band0 * n;
   float wl[NL];
 #pragma unroll
@@ -202,7 +207,7 @@ k_lr_forward(int S, int T, int D, int n, const float* __restrict__ screens,
           n0[l] = ld_at(scr, ro[l] + c0[l]);
           n1[l] = ld_at(scr, ro[l] + c1[l]);
         }
-        float acc = 0.f;
+        float acc = ADD ? o[(size_t)r * n + j] : 0.f;
 #pragma unroll
         for (int l = 0; l < NL; ++l) {
           const float bot = fmaf(cf[l], v1[l] - v0[l], v0[l]);
@@ -220,7 +225,7 @@ k_lr_forward(int S, int T, int D, int n, const float* __restrict__ screens,
       table_row<NL>(tab.up[r], ro);
       table_row<NL>(tab.lo[r], rl);
       table_row<NL>(tab.f[r], fr);
-      float acc = 0.f;
+      float acc = ADD ? o[(size_t)r * n + j] : 0.f;
 #pragma unroll
       for (int l = 0; l < NL; ++l) {
         const float v00 = ld_at(scr, ro[l] + c0[l]), v01 = ld_at(scr, ro[l] + c1[l]);
@@ -234,16 +239,18 @@ k_lr_forward(int S, int T, int D, int n, const float* __restrict__ screens,
   }
 }
 
+// nl <= LM layers of screens whose byte offsets pass 32 bits.
+template <int LM>
 __global__ void __launch_bounds__(256)
-k_lr_forward_any(int L, int S, int T, int D, int n, const float* __restrict__ screens,
+k_lr_forward_any(int L, int nl, int add, int S, int T, int D, int n, const float* __restrict__ screens,
                  const float* __restrict__ w, const long long* __restrict__ fix,
                  float* __restrict__ out) {
-  __shared__ RowTab rt[kLrMaxLayers][kLrBand];
+  __shared__ RowTab rt[LM][kLrBand];
   const int band0 = blockIdx.x * kLrBand;
   const int td = blockIdx.y, b = blockIdx.z;
   const int rows = min(kLrBand, n - band0);
   const long long* fx = fix + (size_t)td * L * 3;
-  for (int k = threadIdx.x; k < L * kLrBand; k += blockDim.x) {
+  for (int k = threadIdx.x; k < nl * kLrBand; k += blockDim.x) {
     const int l = k / kLrBand, r = k % kLrBand;
     const Tap t = lr_tap(fx[3 * l], fx[3 * l + 2], band0 + r, S);
     rt[l][r] = RowTab{t.a0, t.a1, t.f};
@@ -252,15 +259,15 @@ k_lr_forward_any(int L, int S, int T, int D, int n, const float* __restrict__ sc
   const float* scr = screens + (size_t)b * L * S * S;
   float* o = out + ((size_t)b * T * D + td) * n * n + (size_t)band0 * n;
   for (int j = threadIdx.x; j < n; j += blockDim.x) {
-    Tap c[kLrMaxLayers];
+    Tap c[LM];
 #pragma unroll
-    for (int l = 0; l < kLrMaxLayers; ++l)
-      if (l < L) c[l] = lr_tap(fx[3 * l + 1], fx[3 * l + 2], j, S);
+    for (int l = 0; l < LM; ++l)
+      if (l < nl) c[l] = lr_tap(fx[3 * l + 1], fx[3 * l + 2], j, S);
     for (int r = 0; r < rows; ++r) {
-      float acc = 0.f;
+      float acc = add ? o[(size_t)r * n + j] : 0.f;
 #pragma unroll
-      for (int l = 0; l < kLrMaxLayers; ++l) {
-        if (l < L) {
+      for (int l = 0; l < LM; ++l) {
+        if (l < nl) {
           const float* sl = scr + (size_t)l * S * S;
           const RowTab q = rt[l][r];
           const float* s0 = sl + (size_t)q.o0 * S;
@@ -282,7 +289,9 @@ k_lr_forward_any(int L, int S, int T, int D, int n, const float* __restrict__ sc
 // derivative of the bilinear cell the sample lies in). Layers go in groups of
 // NL so that taps and accumulators stay in registers; the band of g is re-read
 // from L2 once per group (NL = 5 takes the 9-layer profile in two; the last
-// group repeats layer L - 1 in its unused places and does not write them).
+// group repeats its last layer in its unused places and does not write them). A
+// launch takes `count` of the L layers, screens, w, fix and partial starting at its
+// first: all of them, but for stacks that pass 32-bit byte offsets.
 // Bounds and row reuse as in the forward: at unit magnification the
 // interpolated value and the column difference of a sample's lower row serve
 // the next pixel. The forward's workload: 1393 us before, 737 us so (issue
@@ -290,7 +299,7 @@ k_lr_forward_any(int L, int S, int T, int D, int n, const float* __restrict__ sc
 constexpr int kLrGroupMax = 5;
 template <int NL>
 __global__ void __launch_bounds__(256, 2)
-k_lr_grad_params(int L, int S, int T, int D, int n, const float* __restrict__ screens,
+k_lr_grad_params(int L, int count, int S, int T, int D, int n, const float* __restrict__ screens,
                  const float* __restrict__ w, const long long* __restrict__ fix,
                  const float* __restrict__ g, float* __restrict__ partial) {
   __shared__ BandTab<NL> tab;
@@ -304,9 +313,9 @@ k_lr_grad_params(int L, int S, int T, int D, int n, const float* __restrict__ sc
   const int nb = gridDim.x;
   float* pp = partial + (((size_t)b * T * D + td) * nb + blockIdx.x) * L * 3;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  for (int l0 = 0; l0 < L; l0 += NL) {
-    const bool unit = all_unit<NL>(fx, l0, L);
-    band_table<NL>(tab, fx, l0, L, S, band0);
+  for (int l0 = 0; l0 < count; l0 += NL) {
+    const bool unit = all_unit<NL>(fx, l0, count);
+    band_table<NL>(tab, fx, l0, count, S, band0);
     __syncthreads();
     float sv[NL], sr[NL], sc[NL];
 #pragma unroll
@@ -316,7 +325,7 @@ k_lr_grad_params(int L, int S, int T, int D, int n, const float* __restrict__ sc
       float cf[NL], fr[NL];
 #pragma unroll
       for (int q = 0; q < NL; ++q) {
-        const int l = min(l0 + q, L - 1);
+        const int l = min(l0 + q, count - 1);
         const Tap c = lr_tap(fx[3 * l + 1], fx[3 * l + 2], j, S);
         c0[q] = 4u * c.a0;
         c1[q] = 4u * c.a1;
@@ -404,7 +413,7 @@ k_lr_grad_params(int L, int S, int T, int D, int n, const float* __restrict__ sc
     __syncthreads();
     if (threadIdx.x < 3 * NL) {
       const int k = threadIdx.x, l = l0 + k / 3;
-      if (l < L) {
+      if (l < count) {
         float s = 0.f;
         for (int q = 0; q < 8; ++q) s += red[q][k];
         pp[3 * l + k % 3] = (k % 3 == 0) ? s : s * w[l];
@@ -414,8 +423,7 @@ k_lr_grad_params(int L, int S, int T, int D, int n, const float* __restrict__ sc
   }
 }
 
-// The same sums, one layer at a time, for screens whose byte offsets pass 32
-// bits.
+// The same sums, one layer at a time, for screens whose byte offsets pass 32 bits.
 __global__ void __launch_bounds__(256)
 k_lr_grad_params_any(int L, int S, int T, int D, int n, const float* __restrict__ screens,
                      const float* __restrict__ w, const long long* __restrict__ fix,
@@ -737,7 +745,7 @@ static int lr_check(const char* who, int B, int L, int S, int T, int D, int n, c
   return PT_OK;
 }
 
-// The screens of one realisation lie within 32-bit byte offsets of their base.
+// L screens lie within 32-bit byte offsets of the first one's base.
 static bool small_offsets(int L, int S) { return 4.0 * L * S * S < 4294967296.0; }
 
 }  // namespace pt
@@ -768,21 +776,30 @@ extern "C" int pt_lr_forward(int B, int L, int S, int T, int D, int n, const dou
   dim3 grid((n + kLrBand - 1) / kLrBand, T * D, B);
   const long long* fx = (const long long*)fix;
   ProfScope ps("k_lr_forward", s);
-  auto go = [&](auto kern) { kern<<<grid, 256, 0, s>>>(S, T, D, n, screens, weights, fx, out); };
-  switch (small_offsets(L, S) ? L : 0) {
-    case 1: go(k_lr_forward<1>); break;
-    case 2: go(k_lr_forward<2>); break;
-    case 3: go(k_lr_forward<3>); break;
-    case 4: go(k_lr_forward<4>); break;
-    case 5: go(k_lr_forward<5>); break;
-    case 6: go(k_lr_forward<6>); break;
-    case 7: go(k_lr_forward<7>); break;
-    case 8: go(k_lr_forward<8>); break;
-    case 9: go(k_lr_forward<9>); break;
-    case 10: go(k_lr_forward<10>); break;
-    default: k_lr_forward_any<<<grid, 256, 0, s>>>(L, S, T, D, n, screens, weights, fx, out);
+  // equal groups of the layers that one launch takes together
+  const bool wide = !small_offsets(1, S);
+  int most = wide ? 8 : kLrTogether;
+  while (!wide && !small_offsets(most, S)) --most;
+  for (int l0 = 0, left = (L + most - 1) / most; left > 0; --left) {
+    const int nl = (L - l0 + left - 1) / left;
+    const float *scr = screens + (size_t)l0 * S * S, *w = weights + l0;
+    auto go = [&](auto first, auto add) {
+      (l0 ? add : first)<<<grid, 256, 0, s>>>(L, S, T, D, n, scr, w, fx + 3 * l0, out);
+    };
+    switch (wide ? 0 : nl) {
+      case 0: {
+        auto kern = nl <= 4 ? k_lr_forward_any<4> : k_lr_forward_any<8>;
+        kern<<<grid, 256, 0, s>>>(L, nl, l0 > 0, S, T, D, n, scr, w, fx + 3 * l0, out);
+        break;
+      }
+#define PT_CASE(k) case k: go(k_lr_forward<k, false>, k_lr_forward<k, true>); break;
+      PT_CASE(1) PT_CASE(2) PT_CASE(3) PT_CASE(4) PT_CASE(5)
+      PT_CASE(6) PT_CASE(7) PT_CASE(8) PT_CASE(9) PT_CASE(10)
+#undef PT_CASE
+    }
+    count_launch_r();
+    l0 += nl;
   }
-  count_launch_r();
   return check_launch("pt_lr_forward");
 }
 
@@ -798,18 +815,29 @@ extern "C" int pt_lr_grad_params(int B, int L, int S, int T, int D, int n, const
   dim3 grid((n + kLrBand - 1) / kLrBand, T * D, B);
   const long long* fx = (const long long*)fix;
   ProfScope ps("k_lr_grad_params", s);
-  auto go = [&](auto kern) {
-    kern<<<grid, 256, 0, s>>>(L, S, T, D, n, screens, weights, fx, grad_out, partial);
-  };
-  // equal groups of at most kLrGroupMax layers
-  const int passes = (L + kLrGroupMax - 1) / kLrGroupMax, nl = (L + passes - 1) / passes;
-  if (!small_offsets(L, S)) go(k_lr_grad_params_any);
-  else if (nl == 1) go(k_lr_grad_params<1>);
-  else if (nl == 2) go(k_lr_grad_params<2>);
-  else if (nl == 3) go(k_lr_grad_params<3>);
-  else if (nl == 4) go(k_lr_grad_params<4>);
-  else go(k_lr_grad_params<5>);
-  count_launch_r();
+  if (!small_offsets(1, S)) {
+    k_lr_grad_params_any<<<grid, 256, 0, s>>>(L, S, T, D, n, screens, weights, fx, grad_out, partial);
+    count_launch_r();
+    return check_launch("pt_lr_grad_params");
+  }
+  // as many layers a launch as lie within 32-bit byte offsets, in equal groups of at
+  // most kLrGroupMax
+  int most = L;
+  while (!small_offsets(most, S)) --most;
+  for (int l0 = 0; l0 < L; l0 += most) {
+    const int count = std::min(most, L - l0);
+    auto go = [&](auto kern) {
+      kern<<<grid, 256, 0, s>>>(L, count, S, T, D, n, screens + (size_t)l0 * S * S, weights + l0,
+                                fx + 3 * l0, grad_out, partial + 3 * l0);
+    };
+    const int passes = (count + kLrGroupMax - 1) / kLrGroupMax, nl = (count + passes - 1) / passes;
+    if (nl == 1) go(k_lr_grad_params<1>);
+    else if (nl == 2) go(k_lr_grad_params<2>);
+    else if (nl == 3) go(k_lr_grad_params<3>);
+    else if (nl == 4) go(k_lr_grad_params<4>);
+    else go(k_lr_grad_params<5>);
+    count_launch_r();
+  }
   return check_launch("pt_lr_grad_params");
 }
 
