@@ -616,9 +616,9 @@ k_lr_grad_unit(int L, int S, int T, int D, int n, int tiles_c, const float* __re
 // Any magnification: the pupil rows that end in screen row r are walked in
 // turn (their count depends only on the row, so the warp does not diverge);
 // KM = ceil(2 / mag) bounds the samples whose footprint covers one pixel along
-// an axis (n >= KM). Entries of unit magnification are left to k_lr_grad_unit
-// with `skip_unit`.
-template <int KM>
+// an axis; a pupil of fewer has SMALL. Entries of unit magnification are left to
+// k_lr_grad_unit with `skip_unit`.
+template <int KM, bool SMALL>
 __global__ void __launch_bounds__(32 * kGsWarps, KM <= 4 ? 7 : 4)
 k_lr_grad_cone(int L, int S, int T, int D, int n, int tiles_c, int skip_unit,
                const float* __restrict__ w, const long long* __restrict__ fix,
@@ -661,7 +661,7 @@ k_lr_grad_cone(int L, int S, int T, int D, int n, int tiles_c, int skip_unit,
         for (int k = 0; k < KM; ++k) {
           const long long dl = p0c + (long long)(xb + k) * m - pf;
           const long long ad = dl < 0 ? -dl : dl;
-          cw[h][k] = ad < kLrOne ? 1.f - (float)ad * 2.3283064365386963e-10f : 0.f;
+          cw[h][k] = ad < kLrOne && (!SMALL || k < n) ? 1.f - (float)ad * 2.3283064365386963e-10f : 0.f;
         }
         p[h] = gi + ((size_t)y * n + xb);
       }
@@ -675,7 +675,7 @@ k_lr_grad_cone(int L, int S, int T, int D, int n, int tiles_c, int skip_unit,
           for (int h = 0; h < 2; ++h) {
             float v = 0.f;
 #pragma unroll
-            for (int k = 0; k < KM; ++k) v = fmaf(cw[h][k], __ldg(p[h] + k), v);
+            for (int k = 0; k < KM; ++k) v = fmaf(cw[h][k], __ldg(p[h] + (SMALL ? min(k, n - 1) : k)), v);
             a0[h] = fmaf(1.f - f, v, a0[h]);
             a1[h] = fmaf(f, v, a1[h]);
             p[h] += n;
@@ -694,35 +694,6 @@ k_lr_grad_cone(int L, int S, int T, int D, int n, int tiles_c, int skip_unit,
   }
   if (accumulate && !any) return;  // nothing to add
   gs_store<kConeRows>(acc, t, S, w[l], accumulate, grad + ((size_t)b * L + l) * S * S);
-}
-
-// Pupils of fewer than eight pixels: a thread a screen pixel, every pupil pixel
-// that may reach it.
-__global__ void __launch_bounds__(256)
-k_lr_grad_tiny(int L, int S, int T, int D, int n, const float* __restrict__ w,
-               const long long* __restrict__ fix, const float* __restrict__ g, int accumulate,
-               float* __restrict__ grad) {
-  const int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= S * S) return;
-  const int l = blockIdx.y, b = blockIdx.z, pr = c / S, pc = c % S;
-  float acc = 0.f;
-  for (int td = 0; td < T * D; ++td) {
-    const long long* fx = fix + ((size_t)td * L + l) * 3;
-    const float* gi = g + ((size_t)b * T * D + td) * n * n;
-    for (int y = 0; y < n; ++y) {
-      const Tap r = lr_tap(fx[0], fx[2], y, S);
-      const float wr = r.a0 == pr ? 1.f - r.f : (r.a1 == pr ? r.f : 0.f);
-      if (wr == 0.f) continue;
-      float v = 0.f;
-      for (int x = 0; x < n; ++x) {
-        const Tap q = lr_tap(fx[1], fx[2], x, S);
-        v = fmaf(q.a0 == pc ? 1.f - q.f : (q.a1 == pc ? q.f : 0.f), gi[y * n + x], v);
-      }
-      acc = fmaf(wr, v, acc);
-    }
-  }
-  float* o = grad + ((size_t)b * L + l) * S * S + c;
-  *o = accumulate ? *o + w[l] * acc : w[l] * acc;
 }
 
 // ----------------------------------------------------------------- host side
@@ -852,12 +823,13 @@ extern "C" int pt_lr_grad_screens(int B, int L, int S, int T, int D, int n, cons
   if (int rc = lr_check("pt_lr_grad_screens", B, L, S, T, D, n, mag)) return rc;
   if (!weights || !fix || !grad_out || !grad_screens)
     return fail(PT_ERR_ARG, "pt_lr_grad_screens: NULL pointer");
-  // which kernels have work: unit magnifications (exactly 1 in fixed point),
-  // and the taps per screen pixel and axis of the others, at most ceil(2 / mag)
+  // which kernels have work: unit magnifications (exactly 1 in fixed point, and two
+  // pixels of the pupil side by side), and the taps per screen pixel and axis of the
+  // others, at most ceil(2 / mag)
   double mmin = 4.0;
   int unit = 0, cone = 0;
   for (int k = 0; k < D * L; ++k) {
-    if (std::llrint(std::ldexp(mag[k], 32)) == kLrOne) {
+    if (n > 1 && std::llrint(std::ldexp(mag[k], 32)) == kLrOne) {
       unit = 1;
     } else {
       cone = 1;
@@ -874,14 +846,6 @@ extern "C" int pt_lr_grad_screens(int B, int L, int S, int T, int D, int n, cons
   };
   const long long* fx = (const long long*)fix;
   ProfScope ps("k_lr_grad_screens", s);
-  if (n < 8) {
-    if ((double)S * S > 2.0e9)
-      return fail(PT_ERR_UNSUPPORTED, "pt_lr_grad_screens: screen too large for a pupil this small");
-    k_lr_grad_tiny<<<dim3((S * S + 255) / 256, L, B), 256, 0, s>>>(L, S, T, D, n, weights, fx,
-                                                                   grad_out, accumulate, grad_screens);
-    count_launch_r();
-    return check_launch("pt_lr_grad_screens");
-  }
   if (unit) {
     k_lr_grad_unit<<<tiles(kUnitRows), 32 * kGsWarps, 0, s>>>(
         L, S, T, D, n, tiles_c, weights, fx, grad_out, accumulate, grad_screens);
@@ -892,10 +856,12 @@ extern "C" int pt_lr_grad_screens(int B, int L, int S, int T, int D, int n, cons
       kern<<<tiles(kConeRows), 32 * kGsWarps, 0, s>>>(L, S, T, D, n, tiles_c, unit, weights, fx,
                                                       grad_out, accumulate, grad_screens);
     };
-    if (km <= 2) go(k_lr_grad_cone<2>);
-    else if (km <= 3) go(k_lr_grad_cone<3>);
-    else if (km <= 4) go(k_lr_grad_cone<4>);
-    else go(k_lr_grad_cone<8>);
+#define PT_CASE(K) go(n < K ? k_lr_grad_cone<K, true> : k_lr_grad_cone<K, false>)
+    if (km <= 2) PT_CASE(2);
+    else if (km <= 3) PT_CASE(3);
+    else if (km <= 4) PT_CASE(4);
+    else PT_CASE(8);
+#undef PT_CASE
     count_launch_r(unit);
   }
   count_launch_r();

@@ -88,3 +88,36 @@ def test_wide_offsets_match_float64(L, S):
     assert rel(out.detach()[0, 0].cpu(), want) < TOL
     assert rel(gw.cpu(), want_w) < TOL_POS
     assert rel(gp.cpu()[0], want_p) < TOL_POS
+
+
+@pytest.mark.parametrize("n", range(1, 8))
+@pytest.mark.parametrize("S,mags", [(31, [1.0, 0.9]), (29, [0.6, 1.0]), (40, [0.4, 0.25]), (66, [1.0, 2.5]), (130, [1.0, 1.0])])
+def test_small_pupils_match_oracle(S, mags, n):
+    screens, w, pos0, mag, n, g = make_case(S + n, 2, 2, S, 3, 2, n, mags)
+    _, gs, gw, gp = run_gpu(screens, w, pos0, mag, n, g)
+    rgs, rgw, rgp = rd.layer_readout_vjp(screens, w.astype(np.float64), pos0, mag, n, g)
+    assert rel(gs, rgs) < TOL
+    assert rel(gw, rgw) < TOL_POS
+    assert rel(gp, rgp) < TOL_POS
+
+
+@pytest.mark.parametrize("S", [300, 46400])   # 46400^2 is beyond a 32-bit pixel index
+def test_tiny_pupil_on_a_wide_screen(S):
+    import torch
+
+    from pyturb_gb300.diff import layer_readout
+
+    screens = torch.zeros((1, 1, S, S), device="cuda", requires_grad=True)
+    w = torch.full((1,), 1.5, device="cuda")
+    pos = torch.tensor([[[[S - 1.75, S - 2.5]]]], dtype=torch.float64, device="cuda")
+    g = torch.arange(1.0, 5.0, device="cuda").reshape(1, 1, 1, 2, 2)
+    out = layer_readout(screens, w, pos, np.ones((1, 1)), 2)
+    (gs,) = torch.autograd.grad(out, screens, g)
+    # samples at rows S - 1.75 and S - 0.75, columns S - 2.5 and S - 1.5 (all weights exact)
+    want = np.zeros((3, 3))
+    for y in range(2):
+        for x in range(2):
+            want[y:y + 2, x:x + 2] += 1.5 * float(g[0, 0, 0, y, x]) * np.outer([0.75, 0.25], [0.5, 0.5])
+    rows, cols = torch.tensor([S - 2, S - 1, 0], device="cuda"), torch.tensor([S - 3, S - 2, S - 1], device="cuda")
+    np.testing.assert_array_equal(gs[0, 0][rows][:, cols].cpu().numpy(), want.astype(np.float32))
+    assert int((gs != 0).sum()) == 9
