@@ -113,12 +113,55 @@ __device__ __forceinline__ void pair_add(float2& a, float x) {
   a.x = t;
 }
 
+// v over the CTA's warps, one sum a lane group: red[warp][i]
+__device__ __forceinline__ void warp_sum(double v, int i, double (*red)[6]) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5][i] = v;
+}
+
+// The six sums of k_adj_params with float64 accumulators, by the whole CTA: for sums
+// that leave the float32 range on the way, or hold an infinity, which the error term
+// of a float pair turns into NaN.
+__device__ __forceinline__ void adj_params_wide(int ns, int F, const float2* spectra, const float2* Z,
+                                             const float2* ph, double (*red)[6]) {
+  const int l = blockIdx.x, p = blockIdx.y;
+  const bool two = 2 * p + 1 < F;
+  const float2 *S = spectra + (size_t)l * ns * ns, *Zp = Z + (size_t)p * ns * ns;
+  const float2 *p0 = ph + ((size_t)l * F + 2 * p) * 2 * ns, *p1 = p0 + 2 * ns;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
+  double acc[6] = {0, 0, 0, 0, 0, 0};
+  for (int kr = warp; kr < ns; kr += warps) {
+    const int nr = kr == 0 ? 0 : ns - kr;
+    const float fxr = (float)signed_freq(kr, ns);
+    for (int kc = lane; kc < ns; kc += 32) {
+      float2 ga, gb;
+      split_pair(Zp[(size_t)kr * ns + kc], Zp[(size_t)nr * ns + (kc == 0 ? 0 : ns - kc)], ga, gb);
+      const float2 s = S[(size_t)kr * ns + kc];
+      const float fyc = (float)signed_freq(kc, ns);
+      const float2 q0 = cmul(cconj(ga), cmul(s, cmul(p0[kr], p0[ns + kc])));
+      acc[0] += q0.x;
+      acc[1] += fxr * q0.y;
+      acc[2] += fyc * q0.y;
+      if (two) {
+        const float2 q1 = cmul(cconj(gb), cmul(s, cmul(p1[kr], p1[ns + kc])));
+        acc[3] += q1.x;
+        acc[4] += fxr * q1.y;
+        acc[5] += fyc * q1.y;
+      }
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < 6; ++i) warp_sum(acc[i], i, red);
+}
+
 // Per (layer, frame pair): [sum Re q, -2 pi w sum fx Im q, -2 pi w sum fy Im q]
 // with q = conj(G_f) S_l Phi_lf, for both frames of the pair, a warp a spectrum
 // row. The sums are kept as float pairs (error-free two-sums) and turned to
 // float64 for the reduction: FP64 adds, at 1/64 of the FP32 rate here, bounded
 // the kernel. 9 layers, 32 frames of 256^2: 258 us with six FP64 adds an
-// element and 256 threads, 53 us so (instruction issue).
+// element and 256 threads, 53 us so (instruction issue). Sums that do not come out
+// finite are formed again by adj_params_wide.
 __global__ void __launch_bounds__(1024)
 k_adj_params(int ns, double df, int L, int F, const float* __restrict__ w,
              const float2* __restrict__ spectra, const float2* __restrict__ Z,
@@ -160,17 +203,20 @@ k_adj_params(int ns, double df, int L, int F, const float* __restrict__ w,
     }
   }
 #pragma unroll
-  for (int i = 0; i < 6; ++i) {
-    double v = (double)acc[i].x + (double)acc[i].y;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    if (lane == 0) red[warp][i] = v;
-  }
+  for (int i = 0; i < 6; ++i) warp_sum((double)acc[i].x + (double)acc[i].y, i, red);
   __syncthreads();
-  if (threadIdx.x < 6) {
-    const int i = threadIdx.x;
+  auto total = [&](int i) {
     double v = 0.0;
     for (int q = 0; q < warps; ++q) v += red[q][i];
+    return v;
+  };
+  if (__syncthreads_or(threadIdx.x < 6 && !isfinite(total(threadIdx.x)))) {
+    adj_params_wide(ns, F, spectra, Z, ph, red);
+    __syncthreads();
+  }
+  if (threadIdx.x < 6) {
+    const int i = threadIdx.x;
+    const double v = total(i);
     const int h = i / 3, c = i % 3;
     const int f = 2 * p + h;
     if (f < F) {
