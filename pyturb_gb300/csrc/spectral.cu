@@ -257,6 +257,9 @@ struct FrameRowArgs {
   int per_layer;
 };
 
+// (PRIME as in k_rows: 64 frames of 9 layers on 64^2, no levels: 28.5 us
+// with, 22.6 us without.)
+template <bool PRIME>
 __global__ void __launch_bounds__(kThreads)
 k_frame_rows(FftDesc d, const float2* __restrict__ tw, FrameRowArgs a, float2* __restrict__ work) {
   extern __shared__ float2 sm[];
@@ -306,7 +309,7 @@ k_frame_rows(FftDesc d, const float2* __restrict__ tw, FrameRowArgs a, float2* _
     bufA[r * vs + ky] = make_float2(h0.x - h1.y, h0.y + h1.x);
   }
   __syncthreads();
-  float2* res = fft_smem(bufA, bufB, d, stw, nrows, vs, 1, false);
+  float2* res = fft_smem<PRIME>(bufA, bufB, d, stw, nrows, vs, 1, false);
   for (int i = threadIdx.x; i < nrows * ns; i += blockDim.x) {
     const int r = i / ns, ky = i % ns;
     const int kx = r == 0 ? kxa : kxb;
@@ -2109,9 +2112,10 @@ extern "C" int pt_frames(const pt_grid* g, int L, const float* spectra, const fl
     }
     if (!uni && !reg && !sum) {
       FrameRowArgs fa{(const float2*)spectra, w.px, w.py, J, nf, f0, per_layer};
-      if (int rc = set_smem(k_frame_rows, rs, "k_frame_rows")) return rc;
+      auto kern = fft_primes(fd) ? k_frame_rows<true> : k_frame_rows<false>;
+      if (int rc = set_smem(kern, rs, "k_frame_rows")) return rc;
       ProfScope ps("k_frame_rows", s);
-      k_frame_rows<<<dim3(ns / 2 + 1, npair), kThreads, rs, s>>>(fd, g->tw, fa, w.img);
+      kern<<<dim3(ns / 2 + 1, npair), kThreads, rs, s>>>(fd, g->tw, fa, w.img);
     }
     count_launch();
     PairStore st{};
