@@ -31,6 +31,31 @@ int check_cuda(cudaError_t e, const char* what) {
 
 int check_launch(const char* what) { return check_cuda(cudaGetLastError(), what); }
 
+// The limit is asked for on each call (0.2 us, as long as setting it takes): a record
+// of our own would go stale with the device's context.
+int allow_smem(const void* kernel, size_t bytes, bool carveout, const char* name) {
+  static std::mutex mu;
+  cudaFuncAttributes have;
+  if (int rc = check_cuda(cudaFuncGetAttributes(&have, kernel), name)) return rc;
+  const auto enough = [&] {
+    return (size_t)have.maxDynamicSharedSizeBytes >= bytes &&
+           (!carveout || have.preferredShmemCarveout == (int)cudaSharedmemCarveoutMaxShared);
+  };
+  if (enough()) return PT_OK;
+  std::lock_guard<std::mutex> lk(mu);
+  if (int rc = check_cuda(cudaFuncGetAttributes(&have, kernel), name)) return rc;
+  if ((size_t)have.maxDynamicSharedSizeBytes < bytes)
+    if (int rc = check_cuda(
+            cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes), name))
+      return rc;
+  if (carveout)
+    if (int rc = check_cuda(cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout,
+                                                 (int)cudaSharedmemCarveoutMaxShared),
+                            name))
+      return rc;
+  return PT_OK;
+}
+
 // ---------------------------------------------------------------- profiling
 struct ProfRec {
   const char* name;

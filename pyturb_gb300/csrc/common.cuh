@@ -19,6 +19,12 @@ int fail(int code, const std::string& msg);
 int check_cuda(cudaError_t e, const char* what);
 int check_launch(const char* what);
 
+// Lets a kernel be launched with `bytes` of dynamic shared memory on the current
+// device (and, with `carveout`, prefers the largest carveout, so that several CTAs fit
+// an SM). The limit is state of the kernel on a device that host threads share: it is
+// only ever raised, never lowered under another thread that is about to launch.
+int allow_smem(const void* kernel, size_t bytes, bool carveout, const char* name);
+
 // ---------------------------------------------------------------- profiling
 // Optional per-kernel timing with CUDA events recorded on the launching
 // stream (pt_prof_enable / pt_prof_report). Off by default: a disabled scope

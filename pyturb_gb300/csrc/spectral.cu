@@ -1057,16 +1057,7 @@ template <class K>
 static int set_smem(K kernel, size_t bytes, const char* name) {
   if (bytes > 227 * 1024)
     return fail(PT_ERR_UNSUPPORTED, std::string(name) + ": grid too large for shared memory");
-  if (bytes > 48 * 1024) {
-    cudaError_t e =
-        cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-    if (e != cudaSuccess) return check_cuda(e, name);
-  }
-  // prefer the largest shared-memory carveout so several CTAs fit per SM
-  cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout,
-                                       (int)cudaSharedmemCarveoutMaxShared);
-  if (e != cudaSuccess) return check_cuda(e, name);
-  return PT_OK;
+  return allow_smem((const void*)kernel, bytes, true, name);
 }
 
 static int check_grid(const pt_grid* g, const char* who) {
