@@ -24,6 +24,7 @@
 #include <stdint.h>
 
 #include <algorithm>
+#include <atomic>
 
 #include "common.cuh"
 #include "tc.cuh"
@@ -401,23 +402,19 @@ extern "C" int pt_ifft2_tc(int ns, const float* in, float* out, int batch, void*
   if ((long long)batch * dft::N > 0x7fffffffLL)
     return fail(PT_ERR_ARG, "pt_ifft2_tc: batch too large");
   cudaStream_t s = (cudaStream_t)stream;
-  static int resident = 0;  // CTAs of k_dft512_tc the device holds at once
+  for (const void* f : {(const void*)k_dft512_tc<false>, (const void*)k_dft512_tc<true>})
+    if (int rc = allow_smem(f, dft::SMEM, true, "pt_ifft2_tc: shared memory")) return rc;
+  int dev = 0;
+  if (int rc = check_cuda(cudaGetDevice(&dev), "pt_ifft2_tc: device")) return rc;
+  static std::atomic<int> known[64];  // CTAs of k_dft512_tc that each device holds at once
+  int resident = dev < 64 ? known[dev].load(std::memory_order_relaxed) : 0;
   if (!resident) {
-    int dev = 0;
-    if (int rc = check_cuda(cudaGetDevice(&dev), "pt_ifft2_tc: device")) return rc;
     cudaDeviceProp prop;
     if (int rc = check_cuda(cudaGetDeviceProperties(&prop, dev), "pt_ifft2_tc: properties")) return rc;
     // CTAs per SM from the SM's shared memory and registers (the occupancy
     // calculator does not follow the carveout preference)
     int per_sm = 4;
     for (const void* f : {(const void*)k_dft512_tc<false>, (const void*)k_dft512_tc<true>}) {
-      if (int rc = check_cuda(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, dft::SMEM),
-                              "pt_ifft2_tc: shared memory"))
-        return rc;
-      if (int rc = check_cuda(cudaFuncSetAttribute(f, cudaFuncAttributePreferredSharedMemoryCarveout,
-                                                   (int)cudaSharedmemCarveoutMaxShared),
-                              "pt_ifft2_tc: carveout"))
-        return rc;
       cudaFuncAttributes fa;
       if (int rc = check_cuda(cudaFuncGetAttributes(&fa, f), "pt_ifft2_tc: attributes")) return rc;
       const size_t per_cta = (size_t)dft::SMEM + fa.sharedSizeBytes + prop.reservedSharedMemPerBlock;
@@ -426,6 +423,7 @@ extern "C" int pt_ifft2_tc(int ns, const float* in, float* out, int batch, void*
     }
     if (per_sm < 1) return fail(PT_ERR_UNSUPPORTED, "pt_ifft2_tc: the kernel does not fit on an SM");
     resident = prop.multiProcessorCount * per_sm;
+    if (dev < 64) known[dev].store(resident, std::memory_order_relaxed);
   }
   const int lines = batch * dft::N;
   const long long img = (long long)dft::N * dft::N;

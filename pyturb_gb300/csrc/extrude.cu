@@ -17,7 +17,6 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
-#include <atomic>
 #include <cmath>
 #include <map>
 #include <vector>
@@ -970,18 +969,7 @@ static size_t step_share_bytes(int W, int J, int modes) {
 template <int RT, int JT>
 static int launch_step(const StepArgs& a, const StepJobs& jobs, const StepJobs& next, cudaStream_t s) {
   const size_t smem = step_smem(a.W, a.K, jobs.n);
-  // the shared-memory limit is a property of the kernel on a device: set once on each
-  static std::atomic<uint64_t> ready{0};
-  int dev = 0;
-  if (int rc = check_cuda(cudaGetDevice(&dev), "k_row_step")) return rc;
-  const uint64_t bit = 1ull << (dev & 63);
-  if (dev > 63 || !(ready.load(std::memory_order_relaxed) & bit)) {
-    if (int rc = check_cuda(cudaFuncSetAttribute(k_row_step<RT, JT>,
-                                                 cudaFuncAttributeMaxDynamicSharedMemorySize, kStepSmem),
-                            "k_row_step"))
-      return rc;
-    if (dev <= 63) ready.fetch_or(bit, std::memory_order_relaxed);
-  }
+  if (int rc = allow_smem((const void*)k_row_step<RT, JT>, smem, false, "k_row_step")) return rc;
   k_row_step<RT, JT><<<(a.W + a.rows - 1) / a.rows, kStepThreads, smem, s>>>(a, jobs, next);
   return PT_OK;
 }

@@ -279,14 +279,7 @@ int tc_gemm_launch(int W, int K, int J, int terms, const uint8_t* At, const uint
   dim3 grid(t.MT, t.nz);
   if (terms == 1) {  // the float32 form's operator correction
     ProfScope ps("k_tc_gemm_lo", s);
-    static bool attr = false;
-    if (!attr) {
-      if (int rc = check_cuda(cudaFuncSetAttribute(k_tc_gemm<1>,
-                                                   cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                   (int)(kTcSmemMax - 1024)), "k_tc_gemm"))
-        return rc;
-      attr = true;
-    }
+    if (int rc = allow_smem((const void*)k_tc_gemm<1>, smem, false, "k_tc_gemm")) return rc;
     k_tc_gemm<1><<<grid, 128, smem, s>>>(W, J, t.NP, t.nkc, t.cps, t.stages, At, Bt, partial);
     count_launch_t();
     *nz_out = t.nz;
@@ -294,24 +287,10 @@ int tc_gemm_launch(int W, int K, int J, int terms, const uint8_t* At, const uint
   }
   ProfScope ps("k_tc_gemm", s);
   if (terms == 2) {
-    static bool attr = false;
-    if (!attr) {
-      if (int rc = check_cuda(cudaFuncSetAttribute(k_tc_gemm<2>,
-                                                   cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                   (int)(kTcSmemMax - 1024)), "k_tc_gemm"))
-        return rc;
-      attr = true;
-    }
+    if (int rc = allow_smem((const void*)k_tc_gemm<2>, smem, false, "k_tc_gemm")) return rc;
     k_tc_gemm<2><<<grid, 128, smem, s>>>(W, J, t.NP, t.nkc, t.cps, t.stages, At, Bt, partial);
   } else {
-    static bool attr = false;
-    if (!attr) {
-      if (int rc = check_cuda(cudaFuncSetAttribute(k_tc_gemm<3>,
-                                                   cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                   (int)(kTcSmemMax - 1024)), "k_tc_gemm"))
-        return rc;
-      attr = true;
-    }
+    if (int rc = allow_smem((const void*)k_tc_gemm<3>, smem, false, "k_tc_gemm")) return rc;
     k_tc_gemm<3><<<grid, 128, smem, s>>>(W, J, t.NP, t.nkc, t.cps, t.stages, At, Bt, partial);
   }
   count_launch_t();
@@ -342,9 +321,7 @@ extern "C" int pt_tc_probe(int N, int K, const uint16_t* A, const uint16_t* B, f
     return fail(PT_ERR_ARG, "pt_tc_probe: N and K must be multiples of 16 in [16, 256]");
   if (!A || !B || !D) return fail(PT_ERR_ARG, "pt_tc_probe: NULL pointer");
   const size_t smem = (size_t)(128 + N) * K * 2 + 1024;
-  if (int rc = check_cuda(cudaFuncSetAttribute(k_tc_probe, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                               (int)smem), "pt_tc_probe"))
-    return rc;
+  if (int rc = allow_smem((const void*)k_tc_probe, smem, false, "pt_tc_probe")) return rc;
   cudaStream_t s = (cudaStream_t)stream;
   k_tc_probe<<<1, 128, smem, s>>>(N, K, A, B, D);
   count_launch_t();

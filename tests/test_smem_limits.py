@@ -17,6 +17,14 @@ def test_one_place_sets_the_limit_of_the_spectral_kernels():
     assert re.search(r"allow_smem\(\(const void\*\)kernel, bytes, true, name\)", source)
 
 
+def test_one_place_sets_the_limit():
+    # a flag of the process behind such a call would skip the second device of a process
+    users = [p.name for p in sorted(CSRC.glob("*.cu*")) if "cudaFuncSetAttribute" in p.read_text()]
+    assert users == ["capi.cu"]
+    helper = (CSRC / "capi.cu").read_text().split("int allow_smem(")[1].split("\n}\n")[0]
+    assert "cudaFuncGetAttributes" in helper and not re.search(r"static (bool|int|size_t)", helper)
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("n", [512, 586])
 def test_threads_of_different_levels_do_not_refuse_each_other(n):
