@@ -381,10 +381,16 @@ class _SynthAdjoint:
                       _ptr(proj), s)
         if part is not None or proj is not None:
             opt = lambda t: None if t is None else _ptr(t)  # noqa: E731
+            scale = self.scale
+            if proj is not None and float(np.float32(scale)) != scale:
+                # the level gradients are float64 and linear in the projections: a factor
+                # that float32 does not hold goes there
+                proj *= scale
+                scale = 1.0
             nbytes = int(_lib.load().pt_synth_adj_levels_workspace_bytes(
                 L, Fc, grid.P if proj is not None else 0))
             work = torch.empty(nbytes, dtype=torch.uint8, device=self.dev)
-            _lib.call("pt_synth_adj_levels", grid.handle, L, Fc, int(f0), self.scale, _ptr(self.w),
+            _lib.call("pt_synth_adj_levels", grid.handle, L, Fc, int(f0), scale, _ptr(self.w),
                       _ptr(self.shr) if proj is not None else None, _ptr(sx), _ptr(sy), opt(proj),
                       opt(part), int(not self.first), opt(self.gw), opt(self.gsh),
                       opt(self.gc) if proj is not None else None, _ptr(work), nbytes, s)
