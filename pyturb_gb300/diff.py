@@ -347,7 +347,7 @@ class _SynthAdjoint:
         self.gsh = new(self.F, self.L, 2) if self.need_p else None
         self.sh = sh_coef
         if sh_coef is not None:
-            self.shr = torch.view_as_real(sh_coef.detach().contiguous())
+            self.shr = torch.view_as_real(sh_coef.detach().resolve_conj().contiguous())
             self.gc = new(self.L, grid.P, 3, 3, 2) if self.need_c else None
         self.first = True
 

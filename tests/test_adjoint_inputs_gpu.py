@@ -1,5 +1,5 @@
 """Inputs of the synthesis adjoint as a caller may give them: a scale that float32
-does not hold."""
+does not hold, level coefficients that are a lazy conjugate."""
 
 import numpy as np
 import pytest
@@ -35,3 +35,10 @@ def test_level_gradients_take_the_scale_in_float64(scale):
     one, _ = level_gradients(1.0)
     got, _ = level_gradients(scale)
     np.testing.assert_allclose(got, scale * one, rtol=0, atol=1e-13 * np.abs(scale * one).max())
+
+
+def test_conjugate_view_of_the_coefficients():
+    shifts, coef = level_gradients(0.5)
+    shifts_c, coef_c = level_gradients(0.5, conj=True)   # conj(conj(c)) as a view
+    np.testing.assert_array_equal(shifts_c, shifts)
+    np.testing.assert_array_equal(coef_c, coef.conj())
