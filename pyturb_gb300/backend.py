@@ -53,8 +53,12 @@ def cuda_device():
 def stream_handle() -> int:
     """cudaStream_t of torch's current stream, so native work orders with torch's."""
     torch = torch_module()
-    # the raw handle, without building a torch.cuda.Stream (several microseconds a call)
-    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device())
+    # the raw handle, without building a torch.cuda.Stream (several microseconds a call);
+    # the function is private to torch, so a release without it takes the public way
+    raw = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+    if raw is None:
+        return torch.cuda.current_stream().cuda_stream
+    return raw(torch.cuda.current_device())
 
 
 def to_numpy(array: Any) -> np.ndarray:
