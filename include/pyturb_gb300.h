@@ -114,9 +114,10 @@ int pt_ifft2_tc(int ns, const float* in, float* out, int batch, void* stream);
  * arrays' addresses (cudaGetSymbolAddress) on the current device; a call made
  * while its stream is captured reuses the address of the last uncaptured call
  * on that device, so make one call on each device before any stream capture.
- * All calls share the arrays, so calls that overlap on the GPU (different
- * streams or threads) race: serialise them, e.g. on one stream. Nothing in
- * the arrays has to start at zero. */
+ * All calls share the arrays: calls from several streams or threads follow one
+ * another on a device (each waits for the one before). The replays of a captured
+ * call do not wait: keep them apart from other uses. Nothing in the arrays has
+ * to start at zero. */
 int pt_ifft2_noalloc(int ns, const float* in, float* out, int batch, void* stream);
 
 /* PhaseScreen.generate(count) (src/pyturb/fourier.py:233-282): coloured

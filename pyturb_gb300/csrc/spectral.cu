@@ -2207,8 +2207,10 @@ extern "C" int pt_boil_step(const pt_grid* g, int L, float* spectra, float* sh_c
 // each device before any stream capture. All calls
 // share the arrays and the last call's contents stay in them; the row pass
 // overwrites every scratch element it later reads and the twiddle table is
-// rewritten by each call, so nothing has to start at zero. Calls that
-// overlap on the GPU (on different streams or threads) race on the arrays.
+// rewritten by each call, so nothing has to start at zero. Calls from several
+// streams or threads follow one another on a device: each waits for an event that
+// the one before records behind its launches. Captured calls carry no event: a
+// replay must not overlap another use of the arrays.
 #include <mutex>
 
 namespace pt {
@@ -2222,7 +2224,23 @@ static __device__ __align__(256) float2 g_noalloc_tw[kNoAllocMaxN];
 struct NoAllocPtrs {
   void* scratch;
   void* tw;
+  cudaEvent_t last;        // behind the last call's launches
+  unsigned long long ctx;  // the context it belongs to
+  bool captured;
 };
+
+// The id of the current context (a device reset gives the device another), or 0.
+static unsigned long long context_id() {
+  using Fn = int (*)(void*, unsigned long long*);
+  static const Fn fn = [] {
+    void* p = nullptr;
+    cudaDriverEntryPointQueryResult q{};
+    const cudaError_t e = cudaGetDriverEntryPointByVersion("cuCtxGetId", &p, 12000, cudaEnableDefault, &q);
+    return e == cudaSuccess && q == cudaDriverEntryPointSuccess ? reinterpret_cast<Fn>(p) : nullptr;
+  }();
+  unsigned long long id = 0;
+  return fn && fn(nullptr, &id) == 0 ? id : 0;
+}
 constexpr int kNoAllocMaxDevices = 64;
 static std::mutex g_noalloc_mu;
 static NoAllocPtrs g_noalloc_ptrs[kNoAllocMaxDevices];
@@ -2236,19 +2254,28 @@ static int noalloc_setup(cudaStream_t s, NoAllocPtrs* out) {
   cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
   if (int rc = check_cuda(cudaStreamIsCapturing(s, &cap), "pt_ifft2_noalloc: cudaStreamIsCapturing"))
     return rc;
-  std::lock_guard<std::mutex> lk(g_noalloc_mu);
   if (cap == cudaStreamCaptureStatusNone || !g_noalloc_ready[dev]) {
-    NoAllocPtrs p{};
+    NoAllocPtrs p = g_noalloc_ptrs[dev];
     if (int rc = check_cuda(cudaGetSymbolAddress(&p.scratch, g_noalloc_scratch),
                             "pt_ifft2_noalloc: cudaGetSymbolAddress(scratch)"))
       return rc;
     if (int rc = check_cuda(cudaGetSymbolAddress(&p.tw, g_noalloc_tw),
                             "pt_ifft2_noalloc: cudaGetSymbolAddress(twiddles)"))
       return rc;
+    const unsigned long long ctx = context_id();
+    if (!p.last || p.ctx != ctx) {  // an event of an earlier context is gone with it
+      if (int rc = check_cuda(cudaEventCreateWithFlags(&p.last, cudaEventDisableTiming),
+                              "pt_ifft2_noalloc: event"))
+        return rc;
+      p.ctx = ctx;
+    } else if (cap == cudaStreamCaptureStatusNone) {
+      if (int rc = check_cuda(cudaStreamWaitEvent(s, p.last, 0), "pt_ifft2_noalloc: event")) return rc;
+    }
     g_noalloc_ptrs[dev] = p;
     g_noalloc_ready[dev] = true;
   }
   *out = g_noalloc_ptrs[dev];
+  out->captured = cap != cudaStreamCaptureStatusNone;
   return PT_OK;
 }
 
@@ -2261,16 +2288,8 @@ __global__ void k_noalloc_twiddles(float2* tw, int n) {
   tw[k] = make_float2((float)c, (float)s);
 }
 
-}  // namespace pt
-
-extern "C" int pt_ifft2_noalloc(int ns, const float* in, float* out, int batch, void* stream) {
-  if (ns < 2 || ns > kNoAllocMaxN)
-    return fail(PT_ERR_ARG, "pt_ifft2_noalloc: ns must be in [2, 1024] (fixed 8 MiB scratch)");
-  if (!in || !out || batch < 0) return fail(PT_ERR_ARG, "pt_ifft2_noalloc: bad arguments");
-  if (batch == 0) return PT_OK;
-  NoAllocPtrs p{};
-  cudaStream_t s = (cudaStream_t)stream;
-  if (int rc = noalloc_setup(s, &p)) return rc;
+static int noalloc_run(int ns, const float* in, float* out, int batch, const NoAllocPtrs& p,
+                       cudaStream_t s) {
   pt_grid g{};  // a stack view over the static arrays: nothing is allocated
   g.ns = ns;
   g.dx = 1.0;
@@ -2307,6 +2326,25 @@ extern "C" int pt_ifft2_noalloc(int ns, const float* in, float* out, int batch, 
     if (int rc = check_launch("pt_ifft2_noalloc")) return rc;
   }
   return PT_OK;
+}
+
+}  // namespace pt
+
+extern "C" int pt_ifft2_noalloc(int ns, const float* in, float* out, int batch, void* stream) {
+  if (ns < 2 || ns > kNoAllocMaxN)
+    return fail(PT_ERR_ARG, "pt_ifft2_noalloc: ns must be in [2, 1024] (fixed 8 MiB scratch)");
+  if (!in || !out || batch < 0) return fail(PT_ERR_ARG, "pt_ifft2_noalloc: bad arguments");
+  if (batch == 0) return PT_OK;
+  NoAllocPtrs p{};
+  cudaStream_t s = (cudaStream_t)stream;
+  std::lock_guard<std::mutex> lk(g_noalloc_mu);  // calls launch, and wait, one after another
+  if (int rc = noalloc_setup(s, &p)) return rc;
+  const int rc = noalloc_run(ns, in, out, batch, p, s);
+  if (!p.captured) {
+    const int er = check_cuda(cudaEventRecord(p.last, s), "pt_ifft2_noalloc: event");
+    if (!rc) return er;
+  }
+  return rc;
 }
 
 // ------------------------------------------------------------------ translate
