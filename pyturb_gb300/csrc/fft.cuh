@@ -302,6 +302,13 @@ inline bool fft_primes(const FftDesc& d) {
   return false;
 }
 
+// Whether a plan has a direct-sum stage.
+inline bool fft_direct(const FftDesc& d) {
+  for (int s = 0; d.M == 0 && s < d.nstages; ++s)
+    if (d.radix[s] > 13) return true;
+  return false;
+}
+
 // The Stockham stages of a length-n transform with the given radices. Kernels for
 // plans without the primes above leave those stages out: they cost 16 to 24 registers
 // a thread even where no stage runs them (100 screens of 144^2: 52 us with, 42 us

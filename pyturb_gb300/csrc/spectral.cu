@@ -938,7 +938,10 @@ k_uniform_sum(int n, const float2* __restrict__ spectra, int L, int F, int run, 
 // both products only on the Nyquist row and column of an even grid, and the CTAs
 // of the last block row make the subharmonic coefficients. Five frames of 9
 // layers on 728^2 took 81.6 us for coefficients, phasor tables and rows in one
-// shared-memory kernel, 44.3 us in this one and the row pass.
+// shared-memory kernel, 44.3 us in this one and the row pass. A CTA walks all
+// layers, so where few CTAs of RB = 4 make the launch its latency counts: RB = 1
+// there (three frames of 16 layers on 200^2, whole call: 55 us with four row pairs
+// a thread, 47 us with one).
 template <int NF, int RB, int CAP>
 __global__ void __launch_bounds__(kSumThreads)
 k_frame_sum(int n, const float2* __restrict__ spectra, const __grid_constant__ FramePrepArgs a,
@@ -997,6 +1000,8 @@ k_frame_sum(int n, const float2* __restrict__ spectra, const __grid_constant__ F
       }
     }
   };
+  // with one row pair a thread, several layers' loads in flight
+#pragma unroll (RB == 1 ? 4 : 1)
   for (int j = 0; j < J; ++j) {
     float2 s[RB], t[RB];
     if (!a.per_layer) load(j, s, t);
@@ -1058,6 +1063,13 @@ static int set_smem(K kernel, size_t bytes, const char* name) {
   if (bytes > 227 * 1024)
     return fail(PT_ERR_UNSUPPORTED, std::string(name) + ": grid too large for shared memory");
   return allow_smem((const void*)kernel, bytes, true, name);
+}
+
+// M of a length 3 M that the Good-Thomas register path takes (M = 64 .. 512), or 0.
+static int gt_m(int ns) {
+  if (ns % 3 != 0) return 0;
+  const int m = ns / 3;
+  return (m >= 64 && m <= 512 && (m & (m - 1)) == 0) ? m : 0;
 }
 
 static int check_grid(const pt_grid* g, const char* who) {
@@ -1262,12 +1274,44 @@ static int launch_frame_rows_reg(const pt_grid* g, const float2* spectra, const 
 }
 
 // ---- frames at arbitrary shifts on other grids
-static bool frames_sum(int ns, int J) { return (ns & (ns - 1)) != 0 && 4 * J <= kShiftTermsMany; }
+// Sums and a row pass against phasor tables and one kernel for sums and rows, by
+// whole calls of F frames, J layers each (us, tables / sums):
+//  - without subharmonic levels the tables' way has no launch more, and wins below
+//    about 1.2e6 pixels: 9 layers, 100^2 F = 5 25 / 33, 288^2 F = 3 40 / 41 and
+//    F = 10 54 / 49, 400^2 F = 5 46 / 51 and F = 10 68 / 58; with the register row pass
+//    of 3 x 2^k below 0.7e6, and on 384^2 never;
+//  - with levels the tables take a launch for the coefficients: below 256^2 they win
+//    from four frames and four layers on (150^2, 9 layers, F = 5 41 / 47; F = 3 41 / 41);
+//  - many layers that take several launches of shifts go to the tables up to 320^2
+//    (60 layers, F = 20: 288^2 293 / 395, 400^2 593 / 471).
+// Bluestein grids have the register transforms in the row pass only: always sums.
+static bool frames_sum(const pt_grid* g, int J, int F) {
+  const int ns = g->ns;
+  if ((ns & (ns - 1)) == 0 || 4 * J > kShiftTermsMany) return false;
+  if (blu_fast(g->desc)) return true;
+  const double px = (double)F * ns * ns;
+  const bool gt = gt_m(ns) != 0;
+  if (J > 40 && ns < 320 && F * J > kShiftTermsMany && !fft_direct(g->desc)) return false;
+  if (g->P == 0) return ns > 512 || px >= (!gt ? 1.2e6 : ns < 256 ? 0.7e6 : 0.0);
+  return !(ns < 256 && F >= 4 && J >= 4 && (px < (gt ? 0.5e6 : 1.2e6) || J > 16));
+}
+// Equally spaced frames pay for their tables and anchors from this many on (the
+// general way below). Whole calls, us, general / equally spaced: 500^2, 16 layers,
+// F = 2 51 / 62; 586^2, 9 layers, F = 5 78 / 72; 150^2, 16 layers, F = 10 47 / 47 and
+// F = 20 62 / 47; without levels 240^2, 3 layers, F = 10 35 / 40 and 9 layers, F = 20
+// 51 / 47; 64^2, 9 layers, F = 16 17 / 23, with levels 25 / 23; 128^2, 9 layers,
+// F = 16 16 / 27 and F = 64 37 / 27.
+static int uniform_from(const pt_grid* g) {
+  const int ns = g->ns;
+  if (blu_fast(g->desc)) return 4;
+  if (ns <= 128 && (ns & (ns - 1)) == 0) return ns == 128 ? 32 : g->P > 0 ? 12 : 24;
+  const double f = std::ceil((g->P > 0 ? 0.3e6 : 0.62e6) / ((double)ns * ns));
+  return (int)std::max(4.0, std::min(24.0, f));
+}
 
-template <int NF, int CAP>
+template <int NF, int CAP, int RB>
 static int frame_sum_t(const pt_grid* g, const float2* spectra, const FramePrepArgs& pa,
                        const double* sx, const double* sy, int f0, float2* img, cudaStream_t s) {
-  constexpr int RB = 4;
   const int n = g->ns;
   auto kern = k_frame_sum<NF, RB, CAP>;
   const size_t smem = (size_t)NF * pa.J * RB * sizeof(float2);
@@ -1286,13 +1330,22 @@ static int frame_sum_t(const pt_grid* g, const float2* spectra, const FramePrepA
 }
 static int launch_frame_sum(const pt_grid* g, const float2* spectra, const FramePrepArgs& pa,
                             const double* sx, const double* sy, int f0, float2* img, cudaStream_t s) {
-  // four frames to a pass over the spectra, but no more than there are
+  // four frames to a pass over the spectra, but no more than there are; one row pair
+  // a thread where four would leave a launch less than two CTAs an SM (over 15 grids
+  // and up to 60 layers: one is 25 to 5% faster below 160 CTAs of four, 1 to 5% to 300,
+  // 1 to 4% slower to 400 and 5 to 12% beyond)
+  const int n = g->ns, nf = pa.F <= 2 ? 2 : 4;
   const bool few = (pa.F + 3) / 4 * 4 * pa.J <= kShiftTermsFew;
-  if (pa.F <= 2)
-    return few ? frame_sum_t<2, kShiftTermsFew>(g, spectra, pa, sx, sy, f0, img, s)
-               : frame_sum_t<2, kShiftTermsMany>(g, spectra, pa, sx, sy, f0, img, s);
-  return few ? frame_sum_t<4, kShiftTermsFew>(g, spectra, pa, sx, sy, f0, img, s)
-             : frame_sum_t<4, kShiftTermsMany>(g, spectra, pa, sx, sy, f0, img, s);
+  const int frames = std::min(pa.F, (few ? kShiftTermsFew : kShiftTermsMany) / pa.J / nf * nf);
+  const bool thin = (long long)((n + kSumThreads - 1) / kSumThreads) * ((n / 2 + 4) / 4) *
+                        ((frames + nf - 1) / nf) < 2 * 152;
+  auto go = [&](auto kern) { return kern(g, spectra, pa, sx, sy, f0, img, s); };
+  constexpr int A = kShiftTermsFew, B = kShiftTermsMany;
+  if (nf == 2)
+    return thin ? go(few ? frame_sum_t<2, A, 1> : frame_sum_t<2, B, 1>)
+                : go(few ? frame_sum_t<2, A, 4> : frame_sum_t<2, B, 4>);
+  return thin ? go(few ? frame_sum_t<4, A, 1> : frame_sum_t<4, B, 1>)
+              : go(few ? frame_sum_t<4, A, 4> : frame_sum_t<4, B, 4>);
 }
 
 // ---- power-of-two dispatch (runtime ns -> template N)
@@ -1433,12 +1486,7 @@ static int default_cols_variant() {
   return v;
 }
 
-// ---- Good-Thomas register path: ns = 3 M, M = 64 .. 512
-static int gt_m(int ns) {
-  if (ns % 3 != 0) return 0;
-  const int m = ns / 3;
-  return (m >= 64 && m <= 512 && (m & (m - 1)) == 0) ? m : 0;
-}
+// ---- Good-Thomas register path
 
 template <int M>
 static int rows_gt_t(const pt_grid* g, const float2* in, int gen, const GenRowArgs& ga, int nimg,
@@ -2044,15 +2092,16 @@ extern "C" int pt_frames(const pt_grid* g, int L, const float* spectra, const fl
     pa.per_layer = per_layer;
     pa.frame0 = f0;
     pa.df = 1.0 / (ns * g->dx);
-    const bool uni = uniform_ok(sx, sy, per_layer, L, f0, nf, ns);
-    const bool uni_reg = uni && (ns == 256 || ns == 512 || ns == 1024);
+    const bool reg_size = ns == 256 || ns == 512 || ns == 1024;
+    const bool uni = (reg_size || nf >= uniform_from(g)) && uniform_ok(sx, sy, per_layer, L, f0, nf, ns);
+    const bool uni_reg = uni && reg_size;
     if (uni_reg) {
       // one prep launch (tables, Nyquist cross, subharmonics) + the fused rows kernel
       if (int rc = launch_uniform_reg_chunk(g, (const float2*)spectra, (const float2*)sh_coef, L,
                                             sx, sy, f0, nf, w, s))
         return rc;
     }
-    const bool reg = !uni && frames_reg(ns, J), sum = !uni && !reg && frames_sum(ns, J);
+    const bool reg = !uni && frames_reg(ns, J), sum = !uni && !reg && frames_sum(g, J, nf);
     if (reg) {
       // phasors, layer sums, row transforms and coefficients in one launch
       if (int rc = launch_frame_rows_reg(g, (const float2*)spectra, pa, sx, sy, f0, w.img, s))
