@@ -74,14 +74,23 @@ static inline int gen_chunk(int ns) {
 // of rows 3072 (more CTAs to fill the last wave; 4096 in brackets: 8 screens of
 // 700^2 81 (83) us, 4 of 1000^2 91 (95) us, three images of 728^2 2 us more) or, of
 // vectors below 320 elements, 2048 (3072 in brackets: 100 screens of 200^2 71 (73)
-// us, 20 of 250^2 42 (44) us, but 64 of 280^2 89 (85) us). A frame pass over `nimg`
-// images takes the 4096 where that makes its rows one wave of three CTAs an SM (five
-// directions on 728^2: 95 us without, 90 us so).
-static inline int rows_per_cta(int nb, int ns = 0, int nimg = 0) {
-  const int r = std::max(1, std::min(16, (nb < 320 ? 2048 : 3072) / nb));
-  const int r2 = std::max(1, std::min(16, 4096 / nb));
-  const auto ctas = [&](int q) { return (long long)((ns + q - 1) / q) * nimg; };
-  return ctas(r) > 3 * 152 && ctas(r2) <= 3 * 152 ? r2 : r;
+// us, 20 of 250^2 42 (44) us, but 64 of 280^2 89 (85) us). 2048 also below 350 CTAs
+// of 3072 (9% faster below 100 such CTAs, 3% at 200 to 300, even at 350, 2 to 5% slower
+// from 400 on, over 20 lengths from 330 to 1500; four screens of 640^2 43 us, 47 us
+// with 3072), and for
+// plans with a direct-sum stage, which want many warps (40 images of 331^2 so 2064 us,
+// with 3072 2585 us). A frame pass takes the 4096 where that makes its rows two to
+// three CTAs an SM in one wave (five directions on 728^2: 95 us without, 90 us so; 64
+// frames of 9 layers on 200^2 64 us and 60 us; below two, 20 frames on 300^2, 55 us
+// without and 60 us so).
+static inline int rows_per_cta(const FftDesc& d, int nimg, bool frames = false) {
+  const int nb = fft_buf_len(d);
+  const auto rows = [&](int elements) { return std::max(1, std::min(16, elements / nb)); };
+  const auto ctas = [&](int r) { return (long long)((d.n + r - 1) / r) * nimg; };
+  const int some = rows(nb < 320 || fft_direct(d) ? 2048 : 3072);
+  if (frames && ctas(some) > 3 * 152 && ctas(rows(4096)) <= 3 * 152 && ctas(rows(4096)) > 2 * 152)
+    return rows(4096);
+  return ctas(some) < 350 ? rows(2048) : some;
 }
 static inline int cols_per_cta(int nb) { return std::max(1, std::min(16, 4096 / nb)); }
 // The shape of a column pass over `nimg` images: where such CTAs would not fill
@@ -1895,7 +1904,7 @@ extern "C" int pt_ifft2(const pt_grid* g, const float* in, float* out, int batch
   if (!work || work_bytes < w.bytes) return fail(PT_ERR_ARG, "pt_ifft2: workspace too small");
   cudaStream_t s = (cudaStream_t)stream;
   const int ns = g->ns, blen = fft_buf_len(g->desc), ch = gen_chunk(ns),
-            rpc = rows_per_cta(blen), C = cols_per_cta(blen);
+            rpc = rows_per_cta(g->desc, std::min(ch, batch)), C = cols_per_cta(blen);
   const size_t rs = rows_smem(ns, blen, rpc), cs = cols_smem(ns, blen, C, 0);
   const bool blu = blu_fast(g->desc);
   if (!pow2_fast(ns) && !blu) {
@@ -1945,7 +1954,7 @@ static int generate_impl(const pt_grid* g, int count, const float* amplitude,
   cudaStream_t s = (cudaStream_t)stream;
   const int n_fft = (count + 1) / 2;
   const int blen = fft_buf_len(g->desc);
-  const int ch = gen_chunk(ns), rpc = rows_per_cta(blen), C = cols_per_cta(blen);
+  const int ch = gen_chunk(ns), rpc = rows_per_cta(g->desc, std::min(ch, n_fft)), C = cols_per_cta(blen);
   const size_t rs = rows_smem(ns, blen, rpc), cs = cols_smem(ns, blen, C, P);
   const bool blu = blu_fast(g->desc);
   if (!pow2_fast(ns) && !gt_m(ns) && !blu) {
@@ -2124,7 +2133,7 @@ extern "C" int pt_frames(const pt_grid* g, int L, const float* spectra, const fl
       } else if (gt_m(ns)) {
         if (int rc = rows_gt(g, w.img, 0, none, npair, w.img, s)) return rc;
       } else {
-        const int rb = fft_buf_len(g->desc), rpc = rows_per_cta(rb, ns, npair);
+        const int rb = fft_buf_len(g->desc), rpc = rows_per_cta(g->desc, npair, true);
         const size_t rsm = rows_smem(ns, rb, rpc);
         if (int rc = set_smem(rows_kernel(g->desc), rsm, "k_rows")) return rc;
         ProfScope ps("k_rows", s);
@@ -2352,7 +2361,7 @@ static int noalloc_run(int ns, const float* in, float* out, int batch, const NoA
       65535, std::max<size_t>(1, kNoAllocScratchBytes / (per * sizeof(float2))));
   k_noalloc_twiddles<<<(ns + 127) / 128, 128, 0, s>>>(g.tw, ns);
   count_launch();
-  const int rpc = rows_per_cta(ns), C = cols_per_cta(ns);  // no Bluestein form here
+  const int rpc = rows_per_cta(g.desc, std::min(chunk, batch)), C = cols_per_cta(ns);  // no Bluestein form here
   const size_t rs = rows_smem(ns, ns, rpc), cs = cols_smem(ns, ns, C, 0);
   if (!pow2_fast(ns)) {
     if (int rc = set_smem(rows_kernel(g.desc), rs, "k_rows")) return rc;
