@@ -451,7 +451,11 @@ __device__ __forceinline__ void anchor_sum(const float2* __restrict__ pj, int Z,
   __syncthreads();
 }
 
-// Few jobs: new row += U d in one launch, a CTA a job and 1024 pixels.
+// new row += U d in one launch, a CTA a job and 1024 pixels: each reads U from L2,
+// and at more than 1024 pixels a job's sums are formed once a CTA, which costs less
+// than a launch of their own. A whole row step of 144 jobs, W = 1449, 64 modes:
+// 105.6 us with a launch for the sums and one for the pixels of eight jobs, 99.6 us
+// so; 24 jobs, W = 200, 32 modes: 38.9 us and 32.7 us.
 template <int R>
 __global__ void __launch_bounds__(1024)
 k_anchor_apply(int W, int cap, int Z, const RingDst dst, const float2* __restrict__ part,
@@ -464,42 +468,6 @@ k_anchor_apply(int W, int cap, int Z, const RingDst dst, const float2* __restric
 #pragma unroll
   for (int i = 0; i < R; ++i) v = fmaf(__ldg(u + (size_t)i * W + w), ds[i], v);
   buf[((size_t)dst.d[j].x * cap + dst.d[j].y) * W + w] += v;
-}
-
-// Many jobs: the sums to d (J, R), then kAddJobs jobs a CTA share each value of
-// U, which a CTA a job would read J times over from L2. 144 jobs, 64 modes, 182
-// shares, W = 1449: 25.8 us with a job's shares scattered over the slices and a
-// lane a share, 15.3 us by k_anchor_apply, 13.5 us so.
-template <int R>
-__global__ void __launch_bounds__(1024)
-k_anchor_sum(int Z, const float2* __restrict__ part, float* __restrict__ d) {
-  __shared__ float ds[R];
-  anchor_sum<R>(part + (size_t)blockIdx.x * Z * R, Z, ds);
-  if (threadIdx.x < R) d[(size_t)blockIdx.x * R + threadIdx.x] = ds[threadIdx.x];
-}
-constexpr int kAddJobs = 8;
-template <int R>
-__global__ void __launch_bounds__(128)
-k_anchor_add(int W, int cap, int J, const RingDst dst, const float* __restrict__ d,
-             const float* __restrict__ u, float* __restrict__ buf) {
-  __shared__ __align__(16) float ds[R][kAddJobs];
-  const int j0 = blockIdx.y * kAddJobs, w = blockIdx.x * 128 + threadIdx.x;
-  for (int e = threadIdx.x; e < R * kAddJobs; e += 128)
-    ds[e % R][e / R] = j0 + e / R < J ? d[(size_t)(j0 + e / R) * R + e % R] : 0.f;
-  __syncthreads();
-  if (w >= W) return;
-  float v[kAddJobs];
-#pragma unroll
-  for (int q = 0; q < kAddJobs; ++q) v[q] = 0.f;
-#pragma unroll 32
-  for (int i = 0; i < R; ++i) {
-    const float ui = __ldg(u + (size_t)i * W + w);
-#pragma unroll
-    for (int q = 0; q < kAddJobs; ++q) v[q] = fmaf(ui, ds[i][q], v[q]);
-  }
-#pragma unroll
-  for (int q = 0; q < kAddJobs; ++q)
-    if (j0 + q < J) buf[((size_t)dst.d[j0 + q].x * cap + dst.d[j0 + q].y) * W + w] += v[q];
 }
 
 // partial[z][j][r] = sum_{k in slice z} M[r][k] X[j][k]
@@ -1512,18 +1480,13 @@ static int extrude_jobs(const char* who, const ExtrudeForm& form, int W, int m,
             }
           }
           {
-            // the operand is spent: its place holds the sums (R <= W modes a job)
-            ProfScope ps("k_anchor_add", s);
-            const dim3 grid((W + 127) / 128, (J + kAddJobs - 1) / kAddJobs);
-            if (R == 32) {
-              k_anchor_sum<32><<<J, 1024, 0, s>>>(nz_a, apart, X);
-              k_anchor_add<32><<<grid, 128, 0, s>>>(W, cap, J, dst, X, an.u, buf);
-            } else {
-              k_anchor_sum<64><<<J, 1024, 0, s>>>(nz_a, apart, X);
-              k_anchor_add<64><<<grid, 128, 0, s>>>(W, cap, J, dst, X, an.u, buf);
-            }
+            ProfScope ps("k_anchor_apply", s);
+            auto go = [&](auto kern) {
+              kern<<<dim3((W + 1023) / 1024, J), 1024, 0, s>>>(W, cap, nz_a, dst, apart, an.u, buf);
+            };
+            if (R == 32) go(k_anchor_apply<32>);
+            else go(k_anchor_apply<64>);
           }
-          count_launch_e();
           count_launch_e(2);
         }
         count_launch_e(form.terms ? 1 : 2);
