@@ -925,9 +925,16 @@ static size_t step_smem(int W, int K, int J) {
   return ((size_t)J * K + (size_t)J * step_rows(W)) * sizeof(float);
 }
 // A row step of at most kStepJobs plain (rows-only, float32) jobs whose operand
-// fits beside the reduction scratch in shared memory.
-static bool step_fits(int W, int K, int J) {
-  return J <= kStepJobs && step_smem(W, K, J) <= kStepSmem;
+// fits beside the reduction scratch in shared memory. Its cost is the staging of the
+// operand in every CTA, J (m + 1) ring rows of at least 0.2 us each; the tiled product
+// costs the same up to 32 jobs. Whole steps in us, k_row_step / tiled: m = 2, 16 jobs:
+// W = 364 15 / 18, W = 728 19 / 21, W = 1000 23 / 27; m = 3, W = 500, 12 jobs 17 / 17
+// and 16 jobs 19 / 17; m = 4, W = 728, 11 jobs 21 / 23 and 14 jobs 25 / 23; m = 8,
+// W = 364, 8 jobs 19 / 19. The anchor of the tiled form takes two launches: m = 8,
+// W = 200, 8 jobs 27 / 29 and 12 jobs 33 / 29; m = 6, W = 500, 11 jobs 32 / 33.
+static bool step_fits(int W, int m, int J, bool anchored) {
+  const int rows = anchored ? 80 : W <= 512 ? 48 : 56;
+  return J <= kStepJobs && J * (m + 1) <= rows && step_smem(W, (m + 1) * W, J) <= kStepSmem;
 }
 static size_t step_share_bytes(int W, int J, int modes) {
   const int ctas = (W + step_rows(W) - 1) / step_rows(W);
@@ -1331,7 +1338,7 @@ static int extrude_jobs(const char* who, const ExtrudeForm& form, int W, int m,
                                  : pt_extrude_workspace_bytes(W, m, sp.n, max_j);
   if (!work || work_bytes < need) return fail(PT_ERR_ARG, std::string(who) + ": workspace too small");
   const int K = (m + 1) * W + sp.n, Kz = m * W + sp.n;
-  if (form.terms == 0 && !form.lo && !form.incr && sp.n == 0 && step_fits(W, K, max_j) &&
+  if (form.terms == 0 && !form.lo && !form.incr && sp.n == 0 && step_fits(W, m, max_j, form.anchor != nullptr) &&
       step_share_bytes(W, max_j, form.anchor ? form.anchor->modes : 0) <= fp32_work(W, m, 0, max_j).partial)
     return step_jobs(who, form, W, m, cap, buf, n_jobs, jobs, noise, work, s);
   const int per_launch = form.terms ? tc_max_jobs(form.terms) : kJobsPerLaunch;
