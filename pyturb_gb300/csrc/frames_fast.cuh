@@ -672,8 +672,7 @@ struct UniformPrep {
   float2* coef;  // (F, P, 9)
   float* mean;   // (F)
   float2* img;   // where the Nyquist cross goes as frame pairs instead of hn, or NULL
-  int N, L, P, F;
-  int nb, run;   // anchors and the frames between them
+  int N, L, P, F, nb;
   int blocks_tab, blocks_nyq;
 };
 
@@ -687,7 +686,7 @@ __global__ void __launch_bounds__(256) k_uniform_prep(UniformPrep a) {
     const int b = bl / L, l = bl % L;
     const uint64_t kk = (uint64_t)(int64_t)signed_freq(k, N);
     if (b < a.nb) {
-      const uint64_t f0 = (uint64_t)b * a.run;
+      const uint64_t f0 = (uint64_t)b * kAnchor;
       a.px0[(size_t)bl * N + k] = phasor_from_fixed(kk * (a.up.ux0[l] + f0 * a.up.dux[l]));
       a.py0[(size_t)bl * N + k] = phasor_from_fixed(kk * (a.up.uy0[l] + f0 * a.up.duy[l]));
     } else {

@@ -861,8 +861,11 @@ k_lgs_zoom_tile(int L, int ns, int n, const int32_t* __restrict__ idx, const flo
 // Y[pair][kx][ky] = H_f0 + i H_f1 for every element off the Nyquist cross (the prep
 // launch writes that), to be transformed in place by the row pass of the grid's
 // form. A thread owns a column ky of the row pair {kx, -kx} and advances the
-// recurrence of k_frame_rows_uniform_reg over `run` frames from its exact anchor:
-// half the sums of a kernel that owns one row, and the transforms get the grid's
+// recurrence of k_frame_rows_uniform_reg over `run` frames, its anchor and its ratio
+// each one rounded phasor of the exact combined phase (as products of two rounded
+// table entries they left the last of 16 frames of white noise on 1000^2 at 1.07e-6,
+// 0.72e-6 so).
+// Half the sums of a kernel that owns one row, and the transforms get the grid's
 // own row pass instead of four rows at a time in shared memory. 64 frames of 9
 // layers on 500^2: 230 us for sums and rows in that kernel, 36 us here and 112 us in
 // the row pass, bound by issue and the stores. Windows of 256 such frames: 500^2
@@ -871,13 +874,14 @@ k_lgs_zoom_tile(int L, int ns, int n, const int32_t* __restrict__ idx, const flo
 constexpr int kSumThreads = 128;
 template <int LM>
 __global__ void __launch_bounds__(kSumThreads, LM <= 4 ? 8 : LM <= 9 ? 5 : 4)
-k_uniform_sum(int n, const float2* __restrict__ spectra, int L, int F, int run, UniformTables ut,
-              float2* __restrict__ img) {
+k_uniform_sum(int n, const float2* __restrict__ spectra, int L, int F, int run,
+              const __grid_constant__ UniformParams up, float2* __restrict__ img) {
   constexpr int LP = (LM + 1) / 2;  // packed layer pairs
   const int ky = blockIdx.x * kSumThreads + threadIdx.x, kx = blockIdx.y;
   const int f0 = blockIdx.z * run, nfr = min(run, F - f0);
   if (ky >= n || 2 * ky == n) return;
   const int nkx = kx ? n - kx : 0, nky = ky ? n - ky : 0;
+  const int kxs = signed_freq(kx, n), kys = signed_freq(ky, n);
   f2x Ax[LP], Ay[LP], Rx[LP], Ry[LP], NRy[LP];
 #pragma unroll
   for (int q = 0; q < LP; ++q) {
@@ -891,9 +895,9 @@ k_uniform_sum(int n, const float2* __restrict__ spectra, int L, int F, int run, 
         const float2 sa = spectra[((size_t)l * n + kx) * n + ky];
         const float2 sb = spectra[((size_t)l * n + nkx) * n + nky];
         const float2 sh = make_float2(0.5f * (sa.x + sb.x), 0.5f * (sa.y - sb.y));
-        const size_t bl = (size_t)blockIdx.z * L + l;
-        const float2 a = cmul(cmul(sh, ut.px0[bl * n + kx]), ut.py0[bl * n + ky]);
-        const float2 r = cmul(ut.rx[(size_t)l * n + kx], ut.ry[(size_t)l * n + ky]);
+        const uint64_t dx = up.dux[l], dy = up.duy[l];
+        const float2 a = cmul(sh, phasor2(kxs, kys, up.ux0[l] + (uint64_t)f0 * dx, up.uy0[l] + (uint64_t)f0 * dy));
+        const float2 r = phasor2(kxs, kys, dx, dy);
         ax[h] = a.x;
         ay[h] = a.y;
         rx[h] = r.x;
@@ -1137,11 +1141,12 @@ static int uniform_reg_rows_t(const pt_grid* g, const float2* spectra, int L, in
   return go(k_frame_rows_uniform_reg<LM, 1024>, 512, 4);
 }
 
-// tables, Nyquist cross and subharmonic coefficients of frames [f0, f0 + nf), an
-// anchor every `run` frames; the cross goes to w.hn, or with `direct` to the images
+// Nyquist cross and subharmonic coefficients of frames [f0, f0 + nf); with `ut` the
+// cross goes to w.hn, and tables with an anchor every kAnchor frames are made for the
+// fused row kernel, else it goes straight to the images
 static int launch_uniform_prep(const pt_grid* g, const float2* spectra, const float2* sh_coef,
-                               int L, const double* sx, const double* sy, int f0, int nf, int run,
-                               bool direct, const SpecWork& w, UniformTables* ut, cudaStream_t s) {
+                               int L, const double* sx, const double* sy, int f0, int nf,
+                               const SpecWork& w, UniformTables* ut, UniformParams* up, cudaStream_t s) {
   const int ns = g->ns;
   const double df = 1.0 / (ns * g->dx);
   UniformPrep a{};
@@ -1158,7 +1163,7 @@ static int launch_uniform_prep(const pt_grid* g, const float2* spectra, const fl
     a.dsx[l] = dx;
     a.dsy[l] = dy;
   }
-  const int nb = (nf + run - 1) / run;
+  const int nb = (nf + kAnchor - 1) / kAnchor;
   float2* ptab = w.px;
   a.px0 = ptab;
   a.py0 = ptab + (size_t)nb * L * ns;
@@ -1176,16 +1181,16 @@ static int launch_uniform_prep(const pt_grid* g, const float2* spectra, const fl
   a.P = g->P;
   a.F = nf;
   a.nb = nb;
-  a.run = run;
-  a.img = direct ? w.img : nullptr;
-  a.blocks_tab = ((nb + 1) * L * ns + 255) / 256;
+  a.img = ut ? nullptr : w.img;
+  a.blocks_tab = ut ? ((nb + 1) * L * ns + 255) / 256 : 0;
   a.blocks_nyq = ns & 1 ? 0 : (2 * ns * ((nf + kNyqGroup - 1) / kNyqGroup) + 255) / 256;
   {
     ProfScope ps("k_uniform_prep", s);
     k_uniform_prep<<<a.blocks_tab + a.blocks_nyq + nf, 256, 0, s>>>(a);
   }
   count_launch();
-  *ut = UniformTables{a.px0, a.py0, a.rx, a.ry};
+  if (ut) *ut = UniformTables{a.px0, a.py0, a.rx, a.ry};
+  if (up) *up = a.up;
   return PT_OK;
 }
 
@@ -1193,8 +1198,7 @@ static int launch_uniform_reg_chunk(const pt_grid* g, const float2* spectra, con
                                     int L, const double* sx, const double* sy, int f0, int nf,
                                     const SpecWork& w, cudaStream_t s) {
   UniformTables ut;
-  if (int rc = launch_uniform_prep(g, spectra, sh_coef, L, sx, sy, f0, nf, kAnchor, false, w, &ut, s))
-    return rc;
+  if (int rc = launch_uniform_prep(g, spectra, sh_coef, L, sx, sy, f0, nf, w, &ut, nullptr, s)) return rc;
   if (L <= 1) return uniform_reg_rows_t<1>(g, spectra, L, nf, ut, w.hn, w.img, s);
   if (L <= 2) return uniform_reg_rows_t<2>(g, spectra, L, nf, ut, w.hn, w.img, s);
   if (L <= 3) return uniform_reg_rows_t<3>(g, spectra, L, nf, ut, w.hn, w.img, s);
@@ -1208,11 +1212,11 @@ static int launch_uniform_reg_chunk(const pt_grid* g, const float2* spectra, con
 // ---- uniform frames on other grids: layer sums, to be transformed by the row pass
 template <int LM>
 static int uniform_sum_t(const pt_grid* g, const float2* spectra, int L, int nf, int run,
-                         const UniformTables& ut, float2* img, cudaStream_t s) {
+                         const UniformParams& up, float2* img, cudaStream_t s) {
   const int n = g->ns;
   ProfScope ps("k_uniform_sum", s);
   k_uniform_sum<LM><<<dim3((n + kSumThreads - 1) / kSumThreads, (n + 1) / 2, (nf + run - 1) / run),
-                      kSumThreads, 0, s>>>(n, spectra, L, nf, run, ut, img);
+                      kSumThreads, 0, s>>>(n, spectra, L, nf, run, up, img);
   count_launch();
   return PT_OK;
 }
@@ -1224,14 +1228,14 @@ static int launch_uniform_sum(const pt_grid* g, const float2* spectra, const flo
   const int n = g->ns, ctas = (n + kSumThreads - 1) / kSumThreads * ((n + 1) / 2);
   const int runs = std::min(8, (1520 + ctas - 1) / ctas);
   const int run = std::max(8, ((nf + runs - 1) / runs + 1) & ~1);
-  UniformTables ut;
-  if (int rc = launch_uniform_prep(g, spectra, sh_coef, L, sx, sy, f0, nf, run, true, w, &ut, s)) return rc;
-  if (L <= 2) return uniform_sum_t<2>(g, spectra, L, nf, run, ut, w.img, s);
-  if (L <= 4) return uniform_sum_t<4>(g, spectra, L, nf, run, ut, w.img, s);
-  if (L <= 6) return uniform_sum_t<6>(g, spectra, L, nf, run, ut, w.img, s);
-  if (L <= 9) return uniform_sum_t<9>(g, spectra, L, nf, run, ut, w.img, s);
-  if (L <= 12) return uniform_sum_t<12>(g, spectra, L, nf, run, ut, w.img, s);
-  return uniform_sum_t<16>(g, spectra, L, nf, run, ut, w.img, s);
+  UniformParams up;
+  if (int rc = launch_uniform_prep(g, spectra, sh_coef, L, sx, sy, f0, nf, w, nullptr, &up, s)) return rc;
+  if (L <= 2) return uniform_sum_t<2>(g, spectra, L, nf, run, up, w.img, s);
+  if (L <= 4) return uniform_sum_t<4>(g, spectra, L, nf, run, up, w.img, s);
+  if (L <= 6) return uniform_sum_t<6>(g, spectra, L, nf, run, up, w.img, s);
+  if (L <= 9) return uniform_sum_t<9>(g, spectra, L, nf, run, up, w.img, s);
+  if (L <= 12) return uniform_sum_t<12>(g, spectra, L, nf, run, up, w.img, s);
+  return uniform_sum_t<16>(g, spectra, L, nf, run, up, w.img, s);
 }
 
 // shifts of global frames [f0, f0 + nf), term by term
