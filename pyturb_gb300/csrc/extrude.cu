@@ -459,12 +459,14 @@ __device__ __forceinline__ void anchor_sum(const float2* __restrict__ pj, int Z,
 template <int R>
 __global__ void __launch_bounds__(1024)
 k_anchor_apply(int W, int cap, int Z, const RingDst dst, const float2* __restrict__ part,
-               const float* __restrict__ u, float* __restrict__ buf) {
+               const float* __restrict__ u, const float* __restrict__ rest, float* __restrict__ buf) {
   __shared__ float ds[R];
   const int j = blockIdx.y, w = blockIdx.x * 1024 + threadIdx.x;
   anchor_sum<R>(part + (size_t)j * Z * R, Z, ds);
   if (w >= W) return;
-  float v = 0.f;
+  // `rest` (J, W), if given, is what float32 dropped of the row: the correction is
+  // smaller than a rounding step, and added to the rounded row it would be lost
+  float v = rest ? rest[(size_t)j * W + w] : 0.f;
 #pragma unroll
   for (int i = 0; i < R; ++i) v = fmaf(__ldg(u + (size_t)i * W + w), ds[i], v);
   buf[((size_t)dst.d[j].x * cap + dst.d[j].y) * W + w] += v;
@@ -729,7 +731,11 @@ __global__ void k_extrude_reduce(int W, int J, int cap, int nsplit, const float*
 // the rings, its warps split K, and the sums end in the ring without slices in
 // memory; the CTA also adds its share of the anchor's projections (a slice of
 // the operand columns, and its own new pixels) and makes its share of the next
-// launch's noise. k_anchor_apply sums the shares and corrects the rows. So the
+// launch's noise. k_anchor_apply sums the shares and corrects the rows, from the new
+// pixels as float pairs: its correction is below a rounding step of the row, and
+// added to rounded pixels it was lost in part, the same part step after step
+// (9-layer frames over 522 rows, four realisations: 4.5e-6 to 8.9e-6, 0.6e-6 to
+// 1.3e-6 so, 0.9e-6 to 2.6e-6 by the tiled product). So the
 // same step takes 11 us + 5 us (both latency: the operand's way through L2, the
 // reduction, the anchor's double-float chains). More than kStepJobs screens, or
 // an operand beyond shared memory, leave the product to the tiled GEMM, which
@@ -795,6 +801,7 @@ struct StepArgs {
   int np2;                     // mode pairs
   int kslice;                  // operand columns of a CTA's anchor share
   float2* part;                // (J, 2 CTAs, 2 np2) shares
+  float* rest;                 // (J, W) what float32 drops of the new rows, for the anchor
 };
 
 template <int RT, int JT>
@@ -803,7 +810,8 @@ k_row_step(const StepArgs a, const StepJobs jobs, const StepJobs next) {
   extern __shared__ float xs[];  // (J, K) operand
   constexpr int NV = RT * JT, NP = (NV + 31) / 32 * 32;
   __shared__ float red[kStepWarps][NP + 1];
-  float* newrow = xs + (size_t)jobs.n * a.K;  // (J, rows)
+  float* newrow = xs + (size_t)jobs.n * a.K;  // (J, rows), then what it drops
+  float* newrest = newrow + (size_t)jobs.n * a.rows;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int W = a.W, K = a.K, J = jobs.n;
   const int rbeg = blockIdx.x * a.rows, rend = min(W, rbeg + a.rows);
@@ -870,11 +878,18 @@ k_row_step(const StepArgs a, const StepJobs jobs, const StepJobs next) {
     if (tid < NV) {
       const int q = tid / JT, j = tid - q * JT, r = r0 + q;
       if (j < J && r < rend) {
-        float v = 0.f;
+        float v = 0.f, rest = 0.f;
+        if (a.th) {
 #pragma unroll
-        for (int w = 0; w < kStepWarps; ++w) v += red[w][tid];
+          for (int w = 0; w < kStepWarps; ++w) two_sum_acc(v, rest, red[w][tid]);
+          a.rest[(size_t)j * W + r] = rest;
+          newrow[j * a.rows + (r - rbeg)] = v;
+          newrest[j * a.rows + (r - rbeg)] = rest;
+        } else {
+#pragma unroll
+          for (int w = 0; w < kStepWarps; ++w) v += red[w][tid];
+        }
         a.buf[((size_t)jobs.screen[j] * a.cap + jobs.head[j]) * W + r] = v;
-        newrow[j * a.rows + (r - rbeg)] = v;
       }
     }
     __syncthreads();
@@ -905,6 +920,10 @@ k_row_step(const StepArgs a, const StepJobs jobs, const StepJobs next) {
         const f2p x2 = pack2(xv, xv);
         if (k >= a.Kz && k < K) c = pfma(ah[u], x2, c);
         else pmac(s, c, ah[u], ah[u] ^ 0x8000000080000000ull, al[u], x2);
+        if (h == 1) {
+          const float rv = newrest[j * a.rows + (k - c0)];
+          c = pfma(ah[u], pack2(rv, rv), c);
+        }
       }
     }
     float s0, s1, e0, e1;
@@ -922,7 +941,7 @@ constexpr int kStepCtas = 152;
 constexpr int kStepSmem = 210 * 1024;
 static int step_rows(int W) { return (W + kStepCtas - 1) / kStepCtas; }
 static size_t step_smem(int W, int K, int J) {
-  return ((size_t)J * K + (size_t)J * step_rows(W)) * sizeof(float);
+  return ((size_t)J * K + 2 * (size_t)J * step_rows(W)) * sizeof(float);
 }
 // A row step of at most kStepJobs plain (rows-only, float32) jobs whose operand
 // fits beside the reduction scratch in shared memory. Its cost is the staging of the
@@ -939,6 +958,10 @@ static bool step_fits(int W, int m, int J, bool anchored) {
 static size_t step_share_bytes(int W, int J, int modes) {
   const int ctas = (W + step_rows(W) - 1) / step_rows(W);
   return (size_t)J * 2 * ctas * modes * sizeof(float2);
+}
+// shares, and what the new rows drop
+static size_t step_bytes(int W, int J, int modes) {
+  return step_share_bytes(W, J, modes) + (size_t)J * W * sizeof(float);
 }
 
 template <int RT, int JT>
@@ -1261,6 +1284,7 @@ static int step_jobs(const char* who, const ExtrudeForm& form, int W, int m, int
   a.np2 = R / 2;
   a.kslice = (K + ctas - 1) / ctas;
   a.part = (float2*)((char*)work + fw.x + fw.lo_tiles);
+  a.rest = (float*)((char*)a.part + step_share_bytes(W, max_j, R));
   {
     const int pairs = launches[0].second.n * ((W + 1) / 2);
     k_step_noise<<<(pairs + 255) / 256, 256, 0, s>>>(launches[0].second, W, noise, nbuf[0]);
@@ -1293,9 +1317,9 @@ static int step_jobs(const char* who, const ExtrudeForm& form, int W, int m, int
       RingDst dst{};
       for (int q = 0; q < cur.n; ++q) dst.d[q] = make_int2(cur.screen[q], cur.head[q]);
       if (R == 32)
-        k_anchor_apply<32><<<grid, 1024, 0, s>>>(W, cap, 2 * ctas, dst, a.part, form.anchor->u, buf);
+        k_anchor_apply<32><<<grid, 1024, 0, s>>>(W, cap, 2 * ctas, dst, a.part, form.anchor->u, a.rest, buf);
       else
-        k_anchor_apply<64><<<grid, 1024, 0, s>>>(W, cap, 2 * ctas, dst, a.part, form.anchor->u, buf);
+        k_anchor_apply<64><<<grid, 1024, 0, s>>>(W, cap, 2 * ctas, dst, a.part, form.anchor->u, a.rest, buf);
       count_launch_e();
     }
     if (int rc = check_launch(who)) return rc;
@@ -1339,7 +1363,7 @@ static int extrude_jobs(const char* who, const ExtrudeForm& form, int W, int m,
   if (!work || work_bytes < need) return fail(PT_ERR_ARG, std::string(who) + ": workspace too small");
   const int K = (m + 1) * W + sp.n, Kz = m * W + sp.n;
   if (form.terms == 0 && !form.lo && !form.incr && sp.n == 0 && step_fits(W, m, max_j, form.anchor != nullptr) &&
-      step_share_bytes(W, max_j, form.anchor ? form.anchor->modes : 0) <= fp32_work(W, m, 0, max_j).partial)
+      step_bytes(W, max_j, form.anchor ? form.anchor->modes : 0) <= fp32_work(W, m, 0, max_j).partial)
     return step_jobs(who, form, W, m, cap, buf, n_jobs, jobs, noise, work, s);
   const int per_launch = form.terms ? tc_max_jobs(form.terms) : kJobsPerLaunch;
   const int jcap = std::min(max_j, per_launch);
@@ -1489,7 +1513,7 @@ static int extrude_jobs(const char* who, const ExtrudeForm& form, int W, int m,
           {
             ProfScope ps("k_anchor_apply", s);
             auto go = [&](auto kern) {
-              kern<<<dim3((W + 1023) / 1024, J), 1024, 0, s>>>(W, cap, nz_a, dst, apart, an.u, buf);
+              kern<<<dim3((W + 1023) / 1024, J), 1024, 0, s>>>(W, cap, nz_a, dst, apart, an.u, nullptr, buf);
             };
             if (R == 32) go(k_anchor_apply<32>);
             else go(k_anchor_apply<64>);
