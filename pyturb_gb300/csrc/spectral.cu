@@ -1348,14 +1348,14 @@ static int frame_sum_t(const pt_grid* g, const float2* spectra, const FramePrepA
 static int launch_frame_sum(const pt_grid* g, const float2* spectra, const FramePrepArgs& pa,
                             const double* sx, const double* sy, int f0, float2* img, cudaStream_t s) {
   // four frames to a pass over the spectra, but no more than there are; one row pair
-  // a thread where four would leave a launch less than two CTAs an SM (over 15 grids
-  // and up to 60 layers: one is 25 to 5% faster below 160 CTAs of four, 1 to 5% to 300,
-  // 1 to 4% slower to 400 and 5 to 12% beyond)
+  // a thread where four would leave less than two CTAs an SM over all launches (15
+  // grids, up to 60 layers: one is 12% faster below 100 CTAs of four, 5% to 300, as
+  // fast at 330, 4% slower to 1000 and 10% beyond; 64 frames of 60 layers on 331^2, in
+  // eight launches of 252 CTAs of four: 822 us with four, 1043 us with one)
   const int n = g->ns, nf = pa.F <= 2 ? 2 : 4;
   const bool few = (pa.F + 3) / 4 * 4 * pa.J <= kShiftTermsFew;
-  const int frames = std::min(pa.F, (few ? kShiftTermsFew : kShiftTermsMany) / pa.J / nf * nf);
   const bool thin = (long long)((n + kSumThreads - 1) / kSumThreads) * ((n / 2 + 4) / 4) *
-                        ((frames + nf - 1) / nf) < 2 * 152;
+                        ((pa.F + nf - 1) / nf) < 2 * 152;
   auto go = [&](auto kern) { return kern(g, spectra, pa, sx, sy, f0, img, s); };
   constexpr int A = kShiftTermsFew, B = kShiftTermsMany;
   if (nf == 2)
