@@ -19,6 +19,7 @@
 #include <algorithm>
 #include <cmath>
 #include <map>
+#include <type_traits>
 #include <vector>
 
 #include <cuda_bf16.h>
@@ -462,14 +463,16 @@ k_anchor_apply(int W, int cap, int Z, const RingDst dst, const float2* __restric
                const float* __restrict__ u, const float* __restrict__ rest, float* __restrict__ buf) {
   __shared__ float ds[R];
   const int j = blockIdx.y, w = blockIdx.x * 1024 + threadIdx.x;
-  anchor_sum<R>(part + (size_t)j * Z * R, Z, ds);
-  if (w >= W) return;
   // `rest` (J, W), if given, is what float32 dropped of the row: the correction is
   // smaller than a rounding step, and added to the rounded row it would be lost
-  float v = rest ? rest[(size_t)j * W + w] : 0.f;
+  float* px = buf + ((size_t)dst.d[j].x * cap + dst.d[j].y) * W + w;
+  const float old = w < W ? *px : 0.f;
+  float v = w < W && rest ? rest[(size_t)j * W + w] : 0.f;
+  anchor_sum<R>(part + (size_t)j * Z * R, Z, ds);
+  if (w >= W) return;
 #pragma unroll
   for (int i = 0; i < R; ++i) v = fmaf(__ldg(u + (size_t)i * W + w), ds[i], v);
-  buf[((size_t)dst.d[j].x * cap + dst.d[j].y) * W + w] += v;
+  *px = old + v;
 }
 
 // partial[z][j][r] = sum_{k in slice z} M[r][k] X[j][k]
@@ -901,7 +904,10 @@ k_row_step(const StepArgs a, const StepJobs jobs, const StepJobs next) {
   const int j = slot % kStepJobs;
   if (j >= J) return;
   const int kb = blockIdx.x * a.kslice, ke = min(K, kb + a.kslice);
-  for (int h = slot / kStepJobs; h < 2; h += slots / kStepJobs) {
+  // share h = 0: the operand columns, 1: the new pixels, each with what it drops (one
+  // loop for both: a step of two jobs, W = 434, 13.7 us, 12.6 us so)
+  auto share = [&](auto h_) {
+    constexpr int h = decltype(h_)::value;
     const int c0 = h == 0 ? kb : K + rbeg, c1 = h == 0 ? ke : K + rend;
     f2p s = 0ull, c = 0ull;
     for (int kc = c0; kc < c1; kc += 8) {  // table entries in flight, 8 columns at a time
@@ -918,11 +924,14 @@ k_row_step(const StepArgs a, const StepJobs jobs, const StepJobs next) {
         if (k >= c1) break;
         const float xv = h == 0 ? xs[j * K + k] : newrow[j * a.rows + (k - c0)];
         const f2p x2 = pack2(xv, xv);
-        if (k >= a.Kz && k < K) c = pfma(ah[u], x2, c);
-        else pmac(s, c, ah[u], ah[u] ^ 0x8000000080000000ull, al[u], x2);
-        if (h == 1) {
-          const float rv = newrest[j * a.rows + (k - c0)];
-          c = pfma(ah[u], pack2(rv, rv), c);
+        if (h == 0 && k >= a.Kz) {
+          c = pfma(ah[u], x2, c);
+        } else {
+          pmac(s, c, ah[u], ah[u] ^ 0x8000000080000000ull, al[u], x2);
+          if (h == 1) {
+            const float rv = newrest[j * a.rows + (k - c0)];
+            c = pfma(ah[u], pack2(rv, rv), c);
+          }
         }
       }
     }
@@ -933,6 +942,10 @@ k_row_step(const StepArgs a, const StepJobs jobs, const StepJobs next) {
     float2* dst = a.part + (((size_t)j * gridDim.x + blockIdx.x) * 2 + h) * 2 * a.np2;
     dst[i0] = make_float2(s0, e0);
     dst[i0 + 16] = make_float2(s1, e1);
+  };
+  for (int h = slot / kStepJobs; h < 2; h += slots / kStepJobs) {
+    if (h == 0) share(std::integral_constant<int, 0>{});
+    else share(std::integral_constant<int, 1>{});
   }
 }
 
