@@ -55,8 +55,9 @@ def stream_handle() -> int:
     torch = torch_module()
     # the raw handle, without building a torch.cuda.Stream (several microseconds a call);
     # the function is private to torch, so a release without it takes the public way
-    raw = getattr(torch._C, "_cuda_getCurrentRawStream", None)
-    if raw is None:
+    try:
+        raw = torch._C._cuda_getCurrentRawStream
+    except AttributeError:
         return torch.cuda.current_stream().cuda_stream
     return raw(torch.cuda.current_device())
 
