@@ -6,6 +6,7 @@
 #include <map>
 #include <mutex>
 #include <string>
+#include <unordered_map>
 #include <vector>
 
 #include "common.cuh"
@@ -31,28 +32,46 @@ int check_cuda(cudaError_t e, const char* what) {
 
 int check_launch(const char* what) { return check_cuda(cudaGetLastError(), what); }
 
-// The limit is asked for on each call (0.2 us, as long as setting it takes): a record
-// of our own would go stale with the device's context.
+unsigned long long context_id() {
+  using Fn = int (*)(void*, unsigned long long*);
+  static const Fn fn = [] {
+    void* p = nullptr;
+    cudaDriverEntryPointQueryResult q{};
+    const cudaError_t e = cudaGetDriverEntryPointByVersion("cuCtxGetId", &p, 12000, cudaEnableDefault, &q);
+    return e == cudaSuccess && q == cudaDriverEntryPointSuccess ? reinterpret_cast<Fn>(p) : nullptr;
+  }();
+  unsigned long long id = 0;
+  return fn && fn(nullptr, &id) == 0 ? id : 0;
+}
+
+// What a thread has seen allowed in a context stays allowed there, so it asks once
+// (0.2 us, as long as setting takes, on each launch otherwise).
 int allow_smem(const void* kernel, size_t bytes, bool carveout, const char* name) {
+  struct Seen {
+    unsigned long long ctx;
+    size_t bytes;
+    bool carveout;
+  };
+  thread_local std::unordered_map<const void*, Seen> seen;
+  const unsigned long long ctx = context_id();
+  Seen& known = seen[kernel];
+  if (ctx && known.ctx == ctx && known.bytes >= bytes && (known.carveout || !carveout)) return PT_OK;
   static std::mutex mu;
+  std::lock_guard<std::mutex> lk(mu);
   cudaFuncAttributes have;
   if (int rc = check_cuda(cudaFuncGetAttributes(&have, kernel), name)) return rc;
-  const auto enough = [&] {
-    return (size_t)have.maxDynamicSharedSizeBytes >= bytes &&
-           (!carveout || have.preferredShmemCarveout == (int)cudaSharedmemCarveoutMaxShared);
-  };
-  if (enough()) return PT_OK;
-  std::lock_guard<std::mutex> lk(mu);
-  if (int rc = check_cuda(cudaFuncGetAttributes(&have, kernel), name)) return rc;
-  if ((size_t)have.maxDynamicSharedSizeBytes < bytes)
+  if ((size_t)have.maxDynamicSharedSizeBytes < bytes) {
     if (int rc = check_cuda(
             cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes), name))
       return rc;
-  if (carveout)
+    have.maxDynamicSharedSizeBytes = (int)bytes;
+  }
+  if (carveout && have.preferredShmemCarveout != (int)cudaSharedmemCarveoutMaxShared)
     if (int rc = check_cuda(cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout,
                                                  (int)cudaSharedmemCarveoutMaxShared),
                             name))
       return rc;
+  known = {ctx, (size_t)have.maxDynamicSharedSizeBytes, carveout};
   return PT_OK;
 }
 

@@ -25,6 +25,9 @@ int check_launch(const char* what);
 // only ever raised, never lowered under another thread that is about to launch.
 int allow_smem(const void* kernel, size_t bytes, bool carveout, const char* name);
 
+// The id of the current context (a device reset gives the device another), or 0.
+unsigned long long context_id();
+
 // ---------------------------------------------------------------- profiling
 // Optional per-kernel timing with CUDA events recorded on the launching
 // stream (pt_prof_enable / pt_prof_report). Off by default: a disabled scope

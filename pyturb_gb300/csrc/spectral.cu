@@ -2296,18 +2296,6 @@ struct NoAllocPtrs {
   bool captured;
 };
 
-// The id of the current context (a device reset gives the device another), or 0.
-static unsigned long long context_id() {
-  using Fn = int (*)(void*, unsigned long long*);
-  static const Fn fn = [] {
-    void* p = nullptr;
-    cudaDriverEntryPointQueryResult q{};
-    const cudaError_t e = cudaGetDriverEntryPointByVersion("cuCtxGetId", &p, 12000, cudaEnableDefault, &q);
-    return e == cudaSuccess && q == cudaDriverEntryPointSuccess ? reinterpret_cast<Fn>(p) : nullptr;
-  }();
-  unsigned long long id = 0;
-  return fn && fn(nullptr, &id) == 0 ? id : 0;
-}
 constexpr int kNoAllocMaxDevices = 64;
 static std::mutex g_noalloc_mu;
 static NoAllocPtrs g_noalloc_ptrs[kNoAllocMaxDevices];
